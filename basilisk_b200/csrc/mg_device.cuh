@@ -272,6 +272,37 @@ __device__ __forceinline__ T relax_value (const bmg_geom & g, long long id, cons
   return nn/d;
 }
 
+/* ---------------------------------------------------------------- */
+/* max reduction                                                     */
+/* ---------------------------------------------------------------- */
+
+/* max that keeps NaN */
+__device__ __forceinline__ double nanmax (double a, double b)
+{
+  return (a > b || a != a) ? a : b;
+}
+
+__device__ __forceinline__ void block_max_atomic (double m, unsigned long long * out)
+{
+  __shared__ double sm[32];
+  const int tid = threadIdx.x + blockDim.x*(threadIdx.y + blockDim.y*threadIdx.z);
+  const int lane = tid & 31;
+  const int nth = blockDim.x*blockDim.y*blockDim.z;
+  for (int o = 16; o > 0; o >>= 1)
+    m = nanmax (m, __shfl_xor_sync (0xffffffffu, m, o));
+  const int warp = tid >> 5;
+  if ((tid & 31) == 0) sm[warp] = m;
+  __syncthreads ();
+  if (warp == 0) {
+    const int nw = (nth + 31) >> 5;
+    double v = lane < nw ? sm[lane] : 0.;
+    for (int o = 16; o > 0; o >>= 1)
+      v = nanmax (v, __shfl_xor_sync (0xffffffffu, v, o));
+    if (lane == 0)
+      atomicMax (out, (unsigned long long) __double_as_longlong (v));
+  }
+}
+
 } // namespace bmgd
 
 #endif

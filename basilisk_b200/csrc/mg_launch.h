@@ -208,19 +208,33 @@ int bmg_launch_bottom (int dim, const bmg_bottom_level * lv, int nlev, bmg_geom 
 /* number of partial sums bmg_launch_sum needs for a level */
 int bmg_sum_partials (int dim, bmg_geom g);
 
-/* implicit viscosity (viscosity.h), 2D and 3D, FP64: one pass of
-   relax_viscosity into w (mode 0: every cell, 1/2: red/black cells), its
-   commit into u (Jacobi average, or the colour's cells), and
-   residual_viscosity with max |res| */
-int bmg_launch_visc_relax (int dim, bmg_geom g, int mode, double * const * u,
-                           double * const * r, double * const * w, const bmg_coef * mu,
-                           bmg_coef rho, double dt, double Delta, cudaStream_t s);
-int bmg_launch_visc_commit (int dim, bmg_geom g, int mode, double * const * u,
-                            double * const * w, cudaStream_t s);
+/* implicit viscosity (viscosity.h), 2D and 3D, FP64 (mg_visc.cu), every
+   component in one launch: a pass of relax_viscosity from in into out with
+   its boundary (mode 0: a Jacobi sweep, 1/2: the red/black cells updated,
+   the others copied), residual_viscosity with max |res|, the restriction
+   and prolongation of a level, and u += da */
+int bmg_launch_visc_pass (int dim, bmg_geom g, int mode, double * const * in, double * const * out,
+                          double * const * r, const bmg_coef * mu, bmg_coef rho, double dt,
+                          double Delta, const bmg_bcdesc * bc, cudaStream_t s);
 int bmg_launch_visc_residual (int dim, bmg_geom g, double * const * u, double * const * r,
                               double * const * res, const bmg_coef * mu, bmg_coef rho,
                               double dt, double Delta, unsigned long long * maxres,
                               cudaStream_t s);
+int bmg_launch_visc_restrict (int dim, bmg_geom gf, bmg_geom gc, double * const * fine,
+                              double * const * coarse, cudaStream_t s);
+int bmg_launch_visc_prolong (int dim, bmg_geom gc, bmg_geom gf, double * const * coarse,
+                             double * const * fine, const bmg_bcdesc * bc, cudaStream_t s);
+int bmg_launch_visc_correct (int dim, bmg_geom g, double * const * u, double * const * da,
+                             const bmg_bcdesc * bc, cudaStream_t s);
+/* levels 0..top of a cycle in one CTA (top at most bmg_visc_bottom_top ()):
+   arrays by level; with restrict_src, res of level top is the restriction
+   of level top + 1 (g and res then have that level too); da: the correction
+   of level top */
+int bmg_visc_bottom_top (int dim);
+int bmg_launch_visc_bottom (int dim, int top, const bmg_geom * g, double * const (* res)[3],
+                            double * const * da, const bmg_coef (* mu)[3], const bmg_coef * rho,
+                            const double * Delta, double dt, int nrelax, int jacobi,
+                            int restrict_src, const bmg_bcdesc * bc, cudaStream_t s);
 
 /* project (poisson.h:468-509): the divergence of a face vector over
    dt Delta, and the face correction uf -= dt alpha grad p of direction e */

@@ -46,8 +46,8 @@ static double * at (const visc_t * v, double * base, int l) { return base + v->g
 
 static double delta (const bmg_grid * g, int l) { return g->L0*(1./(1 << l)); }
 
-/* residual_viscosity (viscosity.h:91-160) after the boundary of u; the
-   maximum goes to g->d_maxres */
+/* residual_viscosity (viscosity.h:91-160), with the boundary of u in place
+   (a cycle's correction writes it); the maximum goes to g->d_maxres */
 static int v_residual (visc_t * v)
 {
   bmg_grid * g = v->g;
@@ -55,7 +55,6 @@ static int v_residual (visc_t * v)
   long long * nl = &v->launches;
   double * u[3], * r[3], * res[3];
   for (int c = 0; c < v->dim; c++) {
-    LV (bmg_launch_apply_bc (v->dim, BMG_ST_F64, g->g64[L], at (v, v->u[c], L), &v->bc[c], 0, g->stream));
     u[c] = at (v, v->u[c], L); r[c] = at (v, v->r[c], L); res[c] = at (v, v->res[c], L);
   }
   CKV (cudaMemsetAsync (g->d_maxres, 0, sizeof (unsigned long long), g->stream));
@@ -64,73 +63,42 @@ static int v_residual (visc_t * v)
   return BMG_OK;
 }
 
-static int v_boundary (visc_t * v, int l)
-{
-  long long * nl = &v->launches;
-  for (int c = 0; c < v->dim; c++)
-    LV (bmg_launch_apply_bc (v->dim, BMG_ST_F64, v->g->g64[l], at (v, v->da[c], l), &v->bc[c], 1,
-                             v->g->stream));
-  return BMG_OK;
-}
-
-/* relax_viscosity (viscosity.h:25-84) on level l */
-static int v_relax (visc_t * v, int l)
-{
-  bmg_grid * g = v->g;
-  long long * nl = &v->launches;
-  double * u[3], * res[3], * w[3];
-  for (int c = 0; c < v->dim; c++) {
-    u[c] = at (v, v->da[c], l); res[c] = at (v, v->res[c], l); w[c] = at (v, v->w[c], l);
-  }
-  if (g->relax == BMG_RELAX_JACOBI) {
-    LV (bmg_launch_visc_relax (v->dim, g->g64[l], 0, u, res, w, v->mu[l], v->rho[l], v->dt,
-                               delta (g, l), g->stream));
-    LV (bmg_launch_visc_commit (v->dim, g->g64[l], 0, u, w, g->stream));
-    return BMG_OK;
-  }
-  for (int colour = 1; colour <= 2; colour++) {
-    if (colour == 2) {
-      int r = v_boundary (v, l);
-      if (r) return r;
-    }
-    LV (bmg_launch_visc_relax (v->dim, g->g64[l], colour, u, res, w, v->mu[l], v->rho[l], v->dt,
-                               delta (g, l), g->stream));
-    LV (bmg_launch_visc_commit (v->dim, g->g64[l], colour, u, w, g->stream));
-  }
-  return BMG_OK;
-}
-
-/* mg_cycle (poisson.h:32-90) on the vector list, minlevel 0 */
+/* mg_cycle (poisson.h:32-90) on the vector list, minlevel 0: the coarse
+   levels in one launch (bmg_launch_visc_bottom), then per level the
+   prolongation and the passes of relax_viscosity (viscosity.h:25-84), which
+   alternate between da and w and write the boundary with the cells */
 static int v_cycle (visc_t * v, int nrelax)
 {
   bmg_grid * g = v->g;
-  const int L = v->L, dim = v->dim;
+  const int L = v->L, dim = v->dim, jacobi = g->relax == BMG_RELAX_JACOBI;
+  const int top = L < bmg_visc_bottom_top (dim) ? L : bmg_visc_bottom_top (dim);
   long long * nl = &v->launches;
-  for (int c = 0; c < dim; c++)
-    for (int l = L - 1; l >= 0; l--)
-      LV (bmg_launch_restrict (dim, BMG_ST_F64, BMG_ST_F64, g->g64[l + 1], g->g64[l],
-                               at (v, v->res[c], l + 1), at (v, v->res[c], l), g->stream));
+  double * res[BMG_MAXLEVEL + 1][3], * cur[3], * oth[3];
+  double Delta[BMG_MAXLEVEL + 1];
   for (int l = 0; l <= L; l++) {
-    for (int c = 0; c < dim; c++) {
-      if (l == 0)
-        LV (bmg_launch_prolong (dim, BMG_ST_F64, BMG_ST_F64, g->g64[l], g->g64[l], NULL,
-                                at (v, v->da[c], l), &v->bc[c], 1, g->stream));
-      else
-        LV (bmg_launch_prolong (dim, BMG_ST_F64, BMG_ST_F64, g->g64[l - 1], g->g64[l],
-                                at (v, v->da[c], l - 1), at (v, v->da[c], l), &v->bc[c], 0,
-                                g->stream));
-    }
-    int r = v_boundary (v, l);
-    if (r) return r;
-    for (int i = 0; i < nrelax; i++) {
-      r = v_relax (v, l);
-      if (!r) r = v_boundary (v, l);
-      if (r) return r;
+    for (int c = 0; c < 3; c++) res[l][c] = c < dim ? at (v, v->res[c], l) : NULL;
+    Delta[l] = delta (g, l);
+  }
+  for (int l = L - 1; l > top; l--)
+    LV (bmg_launch_visc_restrict (dim, g->g64[l + 1], g->g64[l], res[l + 1], res[l], g->stream));
+  for (int c = 0; c < dim; c++) cur[c] = at (v, v->da[c], top);
+  LV (bmg_launch_visc_bottom (dim, top, g->g64, (double * const (*)[3]) res, cur,
+                              (const bmg_coef (*)[3]) v->mu, v->rho, Delta, v->dt, nrelax, jacobi,
+                              top < L, v->bc, g->stream));
+  for (int l = top + 1; l <= L; l++) {
+    double * da[3], * w[3];
+    for (int c = 0; c < dim; c++) { da[c] = at (v, v->da[c], l); w[c] = at (v, v->w[c], l); }
+    LV (bmg_launch_visc_prolong (dim, g->g64[l - 1], g->g64[l], cur, da, v->bc, g->stream));
+    for (int c = 0; c < dim; c++) { cur[c] = da[c]; oth[c] = w[c]; }
+    for (int p = 0; p < (jacobi ? nrelax : 2*nrelax); p++) {
+      LV (bmg_launch_visc_pass (dim, g->g64[l], jacobi ? 0 : 1 + (p & 1), cur, oth, res[l], v->mu[l],
+                                v->rho[l], v->dt, Delta[l], v->bc, g->stream));
+      for (int c = 0; c < dim; c++) { double * t = cur[c]; cur[c] = oth[c]; oth[c] = t; }
     }
   }
-  for (int c = 0; c < dim; c++)
-    LV (bmg_launch_correct (dim, BMG_ST_F64, g->g64[L], g->g64[L], at (v, v->u[c], L),
-                            at (v, v->da[c], L), &v->bc[c], g->stream));
+  double * u[3];
+  for (int c = 0; c < dim; c++) u[c] = at (v, v->u[c], L);
+  LV (bmg_launch_visc_correct (dim, g->g64[L], u, cur, v->bc, g->stream));
   return BMG_OK;
 }
 
@@ -201,19 +169,23 @@ int bmg_viscosity (bmg_grid * g, struct Viscosity p, mgstats * out)
   for (int c = 0; c < v.dim; c++)
     CKV (cudaMemcpyAsync (at (&v, v.r[c], v.L), at (&v, v.u[c], v.L),
                           g->g64[v.L].size*sizeof (double), cudaMemcpyDeviceToDevice, g->stream));
-  /* sum of the r.h.s. (poisson.h:162-167), component by component */
+  /* sum of the r.h.s. (poisson.h:162-167), component by component, each
+     read back in stream order before the next overwrites it */
   for (int c = 0; c < v.dim; c++) {
     LV (bmg_launch_sum (v.dim, g->g64[v.L], at (&v, v.r[c], v.L), g->d_partials, g->npartials,
                         g->d_sum, g->stream));
-    CKV (cudaMemcpyAsync (g->h_pinned + 1, g->d_sum, sizeof (double), cudaMemcpyDeviceToHost,
+    CKV (cudaMemcpyAsync (g->h_pinned + 1 + c, g->d_sum, sizeof (double), cudaMemcpyDeviceToHost,
                           g->stream));
-    CKV (cudaStreamSynchronize (g->stream));
-    s.sum += g->h_pinned[1];
   }
   s.nrelax = p.nrelax > 0 ? p.nrelax : 4;
+  /* the boundary of u as it comes in */
+  for (int c = 0; c < v.dim; c++)
+    LV (bmg_launch_apply_bc (v.dim, BMG_ST_F64, g->g64[v.L], at (&v, v.u[c], v.L), &v.bc[c], 0,
+                             g->stream));
   int r = v_residual (&v);
   if (!r) r = read_max (g, &s.resb);
   if (r) return r;
+  for (int c = 0; c < v.dim; c++) s.sum += g->h_pinned[1 + c];
   double resb = s.resa = s.resb;
   const double tolerance = TOLERANCE;
   int status = BMG_OK;

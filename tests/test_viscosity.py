@@ -208,3 +208,15 @@ def test_viscosity_gpu_matches_oracle(dim, depth, periodic, mu, rho, relax):
     for c, oc in zip(uu, o.get_u()):
         np.testing.assert_array_equal(c.get(), oc)
     g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("relax", ["rbgs", "jacobi"])
+@pytest.mark.parametrize("dim,depth,periodic", [(2, 0, True), (2, 1, False), (2, 5, True), (2, 5, False),
+                                                (2, 6, True), (3, 0, False), (3, 1, True), (3, 3, False),
+                                                (3, 4, True), (3, 5, False)])
+def test_viscosity_gpu_single_cta_levels(dim, depth, periodic, relax):
+    """The levels up to 32^2 (8^3) run in one CTA, the others one pass per
+    launch between two buffers: grids that end inside, at the edge of and
+    one level above that range, bit for bit against the oracle."""
+    test_viscosity_gpu_matches_oracle(dim, depth, periodic, "field", "field", relax)
