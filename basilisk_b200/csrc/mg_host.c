@@ -443,7 +443,7 @@ static int stage_in (bmg_grid * g, const double * values, size_t count, int memo
   return BMG_OK;
 }
 
-static int refresh_bc_ghosts (bmg_grid * g, int h);
+static void bcdesc_of (const bmg_grid * g, const field_t * f, bmg_bcdesc * bc);
 
 int bmg_field_set_level (bmg_grid * g, bmg_scalar s, int level, const double * values,
                          size_t count, int memory)
@@ -456,17 +456,17 @@ int bmg_field_set_level (bmg_grid * g, bmg_scalar s, int level, const double * v
   const double * d;
   int st = stage_in (g, values, count, memory, &d);
   if (st) return st;
-  CL (bmg_launch_pack (g->dim, BMG_ST_F64, g->g64[level], f->face_dim, d, f->lv[level], g->stream));
+  bmg_bcdesc bc;
+  const int ghosts = f->face_dim < 0 && level == g->depth;
+  if (ghosts) bcdesc_of (g, f, &bc);
+  CL (bmg_launch_pack (g->dim, BMG_ST_F64, g->g64[level], f->face_dim, d, f->lv[level],
+                       ghosts ? &bc : NULL, g->stream));
   if (f->face_dim >= 0 && (g->periodic[f->face_dim] || level0_periodic (g, level)))
     /* periodic face vectors: the last face is the image of the first
        (periodic_boundary_level_x copies face vectors, multigrid.h:644-647);
        on a periodic level 0 every neighbour slot takes the cell's value,
        the upper face of every component included (multigrid.h:655-664) */
     CL (bmg_launch_face_wrap (g->dim, g->g64[level], f->face_dim, f->lv[level], g->stream));
-  if (f->face_dim < 0 && level == g->depth) {
-    int r = refresh_bc_ghosts (g, s.i);
-    if (r) return r;
-  }
   CK (cudaStreamSynchronize (g->stream));
   return BMG_OK;
 }

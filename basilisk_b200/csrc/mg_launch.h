@@ -115,8 +115,11 @@ int bmg_launch_apply_bc (int dim, int st, bmg_geom g, void * f,
 int bmg_launch_sum (int dim, bmg_geom g, const double * b, double * partials,
                     int npartials, double * out, cudaStream_t s);
 
+/* bc: the FP64 finest level of a cell field, whose ghost images (of the
+   inhomogeneous conditions) are written too; NULL: none */
 int bmg_launch_pack (int dim, int st, bmg_geom g, int face_dim,
-                     const double * compact, void * padded, cudaStream_t s);
+                     const double * compact, void * padded, const bmg_bcdesc * bc,
+                     cudaStream_t s);
 
 int bmg_launch_unpack (int dim, bmg_geom g, int face_dim, const double * padded,
                        double * compact, cudaStream_t s);
