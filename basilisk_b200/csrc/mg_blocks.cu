@@ -1,0 +1,401 @@
+/*
+ * mg_blocks.cu -- kernels of the solve over a domain decomposed into blocks
+ * (mg_shard.c, the counterpart of grid/multigrid-mpi.h), FP64, 1D to 3D.
+ *
+ * Every launch works on all the blocks of its device, and the thread that
+ * writes a cell writes all its images: the box ghosts of its own block, and
+ * the ghost cells of the neighbouring blocks that mirror it (edges and
+ * corners included), in the neighbour's array -- peer memory over NVLink
+ * when the neighbour lives on another device.  A pass is then one launch
+ * per device with no exchange after it, where it took a launch per block
+ * and one per direction.  No launch reads what it or a launch on another
+ * device writes at the same time: a colour pass reads the other colour only
+ * (n is even, so an image in a neighbour keeps its colour), a Jacobi sweep
+ * and a prolongation write another array than they read, the correction
+ * reads interior cells only.
+ *
+ * The images are those of the exchange they replace (slabs direction by
+ * direction, ghosts of the earlier directions included): the product over
+ * the directions of a cell's own position, its box ghost, its periodic image
+ * in the block, or its image in the neighbour, with the owner's conditions.
+ * Cell updates are relax_value's, k_prolong's, k_restrict's and k_residual's
+ * expressions in their order: bit-identical to one grid over the domain.
+ */
+#include <cuda_runtime.h>
+#include <string.h>
+#include "mg_device.cuh"
+#include "mg_blocks.h"
+
+using namespace bmgd;
+
+namespace {
+
+/* cell q of level l (n = 2^l) in C order */
+template <int DIM>
+__device__ __forceinline__ void cell_at (long long q, int l, int & i, int & j, int & k)
+{
+  const int m = (1 << l) - 1;
+  if (DIM == 1) { i = (int) q; j = k = 0; }
+  else if (DIM == 2) { i = (int) (q >> l); j = (int) q & m; k = 0; }
+  else { i = (int) (q >> (2*l)); j = (int) (q >> l) & m; k = (int) q & m; }
+}
+
+/* write every image of cell (i, j, k) of block b, value v: f (t) is the
+   array of block t that the launch writes, hom the homogeneous conditions
+   (of da) or not (of a) */
+template <int DIM, typename F>
+__device__ __noinline__ void images (const bmg_blk * B, int b, const bmg_geom & g, int i, int j, int k,
+                                     double v, bool hom, F f)
+{
+  const int n = g.n, c[3] = {i, j, k};
+  const bmg_bcdesc & bc = B[b].bc;
+  /* level 0 of a block with periodic directions of its own: every neighbour
+     of the single cell is a copy of it (multigrid.h:655-664) */
+  const bool copies = n == 1 && (bc.periodic[0] || bc.periodic[1] || bc.periodic[2]);
+  /* per direction: the cell itself, and up to two images, each a position
+     and a side s: the box ghost of side s (kind 1), the neighbour on side s
+     (kind 2), or the block's own periodic image (kind 0) */
+  int pos[3][3], sd[3][3], kind[3][3], cnt[3];
+  for (int e = 0; e < 3; e++) {
+    pos[e][0] = c[e]; sd[e][0] = -1; kind[e][0] = 0; cnt[e] = 1;
+    if (e < DIM)
+      for (int hi = 0; hi < 2; hi++)
+        if (c[e] == (hi ? n - 1 : 0)) {
+          const int s = 2*e + (hi ? 0 : 1), t = B[b].nbr[s], q = cnt[e]++;
+          sd[e][q] = s;
+          kind[e][q] = t >= 0 ? 2 : bc.periodic[e] ? 0 : 1;
+          /* beyond the side for a box ghost, across for an image */
+          pos[e][q] = (kind[e][q] == 1) == (hi == 1) ? n : -1;
+        }
+  }
+  for (int x = 0; x < cnt[0]; x++)
+    for (int y = 0; y < cnt[1]; y++)
+      for (int z = 0; z < cnt[2]; z++) {
+        if (x == 0 && y == 0 && z == 0) continue;
+        const int at[3] = {x, y, z};
+        double r = v;
+        int t = b;
+        for (int e = 0; e < DIM; e++) {
+          const int q = at[e], s = sd[e][q];
+          if (kind[e][q] == 2) t = B[t].nbr[s];
+          else if (kind[e][q] == 1 && !copies) {
+            if (hom) r = bc.type[s] == 1 /* BMG_DIRICHLET */ ? r*(-1.) : r;
+            else {
+              const double w = bc_data<DIM> (bc, s, n, i, j, k);
+              r = bc.type[s] == 1 ? 2.*(w) - r : bc.Delta*(w) + r;
+            }
+          }
+        }
+        f (t)[cidx<DIM> (g, pos[0][x], pos[1][y], pos[2][z])] = r;
+      }
+}
+
+template <int DIM, typename F>
+__device__ __forceinline__ void put (const bmg_blk * B, int b, const bmg_geom & g, int i, int j, int k,
+                                     double v, bool hom, F f)
+{
+  f (b)[cidx<DIM> (g, i, j, k)] = v;
+  if (on_boundary<DIM> (g.n, i, j, k)) images<DIM> (B, b, g, i, j, k, v, hom, f);
+}
+
+/* the update of one cell of block b of level l */
+template <int DIM>
+__device__ __forceinline__ double update (const bmg_blk_level & L, const bmg_geom & g, long long id,
+                                          const double * in, double D2)
+{
+  return relax_value<DIM, double> (g, id, in, L.res, coef_of<double> (L.alpha[0]),
+                                   coef_of<double> (L.alpha[1]), coef_of<double> (L.alpha[2]),
+                                   coef_of<double> (L.lambda), D2);
+}
+
+/* cell h of the n/2 of one colour in a row */
+template <int DIM>
+__device__ __forceinline__ void colour_cell (long long q, int l, int colour, int & i, int & j, int & k)
+{
+  const int lh = l - 1, m = (1 << l) - 1, h = (int) q & ((1 << lh) - 1);
+  const long long row = q >> lh;
+  if (DIM == 1) { i = 2*h + colour; j = k = 0; }
+  else if (DIM == 2) { i = (int) row; j = 2*h + ((colour + i) & 1); k = 0; }
+  else { i = (int) (row >> l); j = (int) row & m; k = 2*h + ((colour + i + j) & 1); }
+}
+
+/* blockIdx.y: the block (of the launch's own); a thread per cell of the
+   colour, or per cell (Jacobi) */
+template <int DIM, int MODE>
+__global__ void k_blocks_relax (bmg_geom g, int l, bmg_blocks B, double Delta, int odd)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  const long long q = (long long) blockIdx.x*blockDim.x + threadIdx.x;
+  const long long cells = 1LL << (DIM*l);
+  if (q >= (MODE == BMG_SWEEP_JACOBI ? cells : cells/2)) return;
+  const int b = B.mine[blockIdx.y];
+  const bmg_blk_level * lv = B.lv + (long long) l*B.nb;
+  const bmg_blk_level & L = lv[b];
+  int i, j, k;
+  if (MODE == BMG_SWEEP_JACOBI) cell_at<DIM> (q, l, i, j, k);
+  else colour_cell<DIM> (q, l, MODE == BMG_SWEEP_RED ? 0 : 1, i, j, k);
+  const long long id = cidx<DIM> (g, i, j, k);
+  if (MODE == BMG_SWEEP_JACOBI) {
+    const double * in = odd ? L.da2 : L.da;
+    const double c = update<DIM> (L, g, id, in, Delta*Delta);
+    put<DIM> (B.blk, b, g, i, j, k, (in[id] + 2.*c)/3., true,
+              [=] (int t) { return odd ? lv[t].da : lv[t].da2; });
+  }
+  else
+    put<DIM> (B.blk, b, g, i, j, k, update<DIM> (L, g, id, L.da, Delta*Delta), true,
+              [=] (int t) { return lv[t].da; });
+}
+
+/* bilinear (multigrid-common.h:124-140) in k_prolong's expression and order */
+template <int DIM>
+__device__ __forceinline__ double bilinear (const bmg_geom & gc, const double * s, int i, int j, int k)
+{
+  const int pi = i >> 1, cx = (i & 1) ? 1 : -1, pj = j >> 1, cy = (j & 1) ? 1 : -1;
+  if (DIM == 1)
+    return (3.*s[cidx<1> (gc, pi, 0, 0)] + s[cidx<1> (gc, pi + cx, 0, 0)])/4.;
+  if (DIM == 2)
+    return (9.*s[cidx<2> (gc, pi, pj, 0)] +
+            3.*(s[cidx<2> (gc, pi + cx, pj, 0)] + s[cidx<2> (gc, pi, pj + cy, 0)]) +
+            s[cidx<2> (gc, pi + cx, pj + cy, 0)])/16.;
+  const int pk = k >> 1, cz = (k & 1) ? 1 : -1;
+  return (27.*s[cidx<3> (gc, pi, pj, pk)] +
+          9.*(s[cidx<3> (gc, pi + cx, pj, pk)] + s[cidx<3> (gc, pi, pj + cy, pk)] +
+              s[cidx<3> (gc, pi, pj, pk + cz)]) +
+          3.*(s[cidx<3> (gc, pi + cx, pj + cy, pk)] + s[cidx<3> (gc, pi + cx, pj, pk + cz)] +
+              s[cidx<3> (gc, pi, pj + cy, pk + cz)]) +
+          s[cidx<3> (gc, pi + cx, pj + cy, pk + cz)])/64.;
+}
+
+template <int DIM>
+__global__ void k_blocks_prolong (bmg_geom gc, bmg_geom g, int l, bmg_blocks B, int odd)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  const long long q = (long long) blockIdx.x*blockDim.x + threadIdx.x;
+  if (q >= 1LL << (DIM*l)) return;
+  const int b = B.mine[blockIdx.y];
+  const bmg_blk_level * lv = B.lv + (long long) l*B.nb;
+  int i, j, k;
+  cell_at<DIM> (q, l, i, j, k);
+  double v = 0.;
+  if (gc.n) {
+    const bmg_blk_level & C = (lv - B.nb)[b];
+    v = bilinear<DIM> (gc, odd ? C.da2 : C.da, i, j, k);
+  }
+  put<DIM> (B.blk, b, g, i, j, k, v, true, [=] (int t) { return lv[t].da; });
+}
+
+/* restriction_average (multigrid-common.h:26-32) in foreach_child order */
+template <int DIM>
+__device__ __forceinline__ double mean (const bmg_geom & gf, const double * f, int i, int j, int k)
+{
+  double sum = 0.;
+#pragma unroll
+  for (int a = 0; a < 2; a++)
+#pragma unroll
+    for (int b = 0; b < (DIM > 1 ? 2 : 1); b++)
+#pragma unroll
+      for (int d = 0; d < (DIM > 2 ? 2 : 1); d++)
+        sum += f[cidx<DIM> (gf, 2*i + a, 2*j + b, 2*k + d)];
+  return sum/(double) (1 << DIM);
+}
+
+template <int DIM>
+__global__ void k_blocks_restrict (bmg_geom gf, bmg_geom g, int l, bmg_blocks B)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  const long long q = (long long) blockIdx.x*blockDim.x + threadIdx.x;
+  if (q >= 1LL << (DIM*l)) return;
+  const bmg_blk_level * lv = B.lv + (long long) l*B.nb + B.mine[blockIdx.y];
+  int i, j, k;
+  cell_at<DIM> (q, l, i, j, k);
+  lv->res[cidx<DIM> (g, i, j, k)] = mean<DIM> (gf, lv[B.nb].res, i, j, k);
+}
+
+template <int DIM>
+__global__ void k_blocks_correct (bmg_geom g, int l, bmg_blocks B, int odd)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  const long long q = (long long) blockIdx.x*blockDim.x + threadIdx.x;
+  if (q >= 1LL << (DIM*l)) return;
+  const int b = B.mine[blockIdx.y];
+  const bmg_blk_level & L = B.lv[(long long) l*B.nb + b];
+  int i, j, k;
+  cell_at<DIM> (q, l, i, j, k);
+  const long long id = cidx<DIM> (g, i, j, k);
+  const bmg_blk * blk = B.blk;
+  put<DIM> (blk, b, g, i, j, k, blk[b].a[id] + (odd ? L.da2 : L.da)[id], false,
+            [=] (int t) { return blk[t].a; });
+}
+
+/* k_residual's expression and order (poisson.h:373-389) */
+template <int DIM, bool POW2>
+__global__ void k_blocks_residual (bmg_geom g, int l, bmg_blocks B, double Delta,
+                                   unsigned long long * maxres)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  const long long q = (long long) blockIdx.x*blockDim.x + threadIdx.x;
+  double m = 0.;
+  const double rD = 1./Delta;
+  if (q < 1LL << (DIM*l)) {
+    const int b = B.mine[blockIdx.y];
+    const bmg_blk_level & L = B.lv[(long long) l*B.nb + b];
+    int i, j, k;
+    cell_at<DIM> (q, l, i, j, k);
+    const long long id = cidx<DIM> (g, i, j, k);
+    const double * a = B.blk[b].a, ac = a[id];
+    const Coef<double> lam = coef_of<double> (L.lambda);
+    double r = B.blk[b].b[id] - lam.at (id)*ac;
+#pragma unroll
+    for (int e = 0; e < DIM; e++) {
+      const Coef<double> al = coef_of<double> (L.alpha[e]);
+      const long long s = cstride<DIM> (g, e);
+      r += over_delta<POW2> (al.at (id)*over_delta<POW2> (ac - a[id - s], Delta, rD) -
+                             al.at (id + s)*over_delta<POW2> (a[id + s] - ac, Delta, rD), Delta, rD);
+    }
+    L.res[id] = r;
+    m = fabs (r);
+  }
+  block_max_atomic (m, maxres);
+}
+
+struct BottomParams {
+  bmg_geom g[BMG_MAXLEVEL + 1];
+  double Delta[BMG_MAXLEVEL + 1];
+  bmg_blocks B;
+  int lo, hi, nrelax, restrict_src;
+};
+
+/* the coarse levels of all the blocks in one CTA: a barrier between passes
+   instead of a launch (its own global writes are visible to the CTA after
+   the barrier, and its L1 serves them).  Bound: the latency of a pass. */
+template <int DIM>
+__global__ void __launch_bounds__ (1024, 1) k_blocks_bottom (const __grid_constant__ BottomParams P)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  const bmg_blocks & B = P.B;
+  for (int l = P.restrict_src ? P.hi : P.hi - 1; l >= P.lo; l--) {
+    const int cells = 1 << (DIM*l);
+    for (int q = threadIdx.x; q < cells*B.m; q += blockDim.x) {
+      const bmg_blk_level * lv = B.lv + (long long) l*B.nb + B.mine[q >> (DIM*l)];
+      int i, j, k;
+      cell_at<DIM> (q & (cells - 1), l, i, j, k);
+      lv->res[cidx<DIM> (P.g[l], i, j, k)] = mean<DIM> (P.g[l + 1], lv[B.nb].res, i, j, k);
+    }
+    __syncthreads ();
+  }
+  for (int l = P.lo; l <= P.hi; l++) {
+    const bmg_geom & g = P.g[l];
+    const bmg_blk_level * lv = B.lv + (long long) l*B.nb;
+    const int cells = 1 << (DIM*l);
+    auto da = [=] (int t) { return lv[t].da; };
+    for (int q = threadIdx.x; q < cells*B.m; q += blockDim.x) {
+      const int b = B.mine[q >> (DIM*l)];
+      int i, j, k;
+      cell_at<DIM> (q & (cells - 1), l, i, j, k);
+      const double v = l == P.lo ? 0. : bilinear<DIM> (P.g[l - 1], (lv - B.nb)[b].da, i, j, k);
+      put<DIM> (B.blk, b, g, i, j, k, v, true, da);
+    }
+    __syncthreads ();
+    const double D2 = P.Delta[l]*P.Delta[l];
+    for (int p = 0; p < 2*P.nrelax; p++) {
+      for (int q = threadIdx.x; q < (cells >> 1)*B.m; q += blockDim.x) {
+        const int b = B.mine[q >> (DIM*l - 1)];
+        int i, j, k;
+        colour_cell<DIM> (q & ((cells >> 1) - 1), l, p & 1, i, j, k);
+        const long long id = cidx<DIM> (g, i, j, k);
+        put<DIM> (B.blk, b, g, i, j, k, update<DIM> (lv[b], g, id, lv[b].da, D2), true, da);
+      }
+      __syncthreads ();
+    }
+  }
+}
+
+#define NT 256
+
+dim3 grid_of (long long threads, int m) { return dim3 ((unsigned) ((threads + NT - 1)/NT), m, 1); }
+
+int status_of (cudaError_t launched)
+{
+  const cudaError_t e = cudaGetLastError ();
+  return launched != cudaSuccess ? (int) launched : (int) e;
+}
+
+template <int DIM>
+cudaError_t relax_dim (int mode, int odd, bmg_geom g, int l, bmg_blocks B, double Delta, cudaStream_t s)
+{
+  const long long cells = 1LL << (DIM*l);
+  if (mode == BMG_SWEEP_JACOBI)
+    return pdl_launch (k_blocks_relax<DIM, BMG_SWEEP_JACOBI>, grid_of (cells, B.m), dim3 (NT), 0, s, g, l, B, Delta, odd);
+  if (mode == BMG_SWEEP_RED)
+    return pdl_launch (k_blocks_relax<DIM, BMG_SWEEP_RED>, grid_of (cells/2, B.m), dim3 (NT), 0, s, g, l, B, Delta, 0);
+  return pdl_launch (k_blocks_relax<DIM, BMG_SWEEP_BLACK>, grid_of (cells/2, B.m), dim3 (NT), 0, s, g, l, B, Delta, 0);
+}
+
+} // namespace
+
+extern "C" {
+
+int bmg_blocks_relax (int dim, int mode, int odd, bmg_geom g, int l, bmg_blocks B, double Delta,
+                      cudaStream_t s)
+{
+  if (l < 1) return (int) cudaErrorInvalidValue;
+  return status_of (dim == 1 ? relax_dim<1> (mode, odd, g, l, B, Delta, s)
+                    : dim == 2 ? relax_dim<2> (mode, odd, g, l, B, Delta, s)
+                    : relax_dim<3> (mode, odd, g, l, B, Delta, s));
+}
+
+int bmg_blocks_prolong (int dim, int odd, bmg_geom gc, bmg_geom g, int l, bmg_blocks B, cudaStream_t s)
+{
+  const dim3 gb = grid_of (1LL << (dim*l), B.m);
+  return status_of (dim == 1 ? pdl_launch (k_blocks_prolong<1>, gb, dim3 (NT), 0, s, gc, g, l, B, odd)
+                    : dim == 2 ? pdl_launch (k_blocks_prolong<2>, gb, dim3 (NT), 0, s, gc, g, l, B, odd)
+                    : pdl_launch (k_blocks_prolong<3>, gb, dim3 (NT), 0, s, gc, g, l, B, odd));
+}
+
+int bmg_blocks_restrict (int dim, bmg_geom gf, bmg_geom g, int l, bmg_blocks B, cudaStream_t s)
+{
+  const dim3 gb = grid_of (1LL << (dim*l), B.m);
+  return status_of (dim == 1 ? pdl_launch (k_blocks_restrict<1>, gb, dim3 (NT), 0, s, gf, g, l, B)
+                    : dim == 2 ? pdl_launch (k_blocks_restrict<2>, gb, dim3 (NT), 0, s, gf, g, l, B)
+                    : pdl_launch (k_blocks_restrict<3>, gb, dim3 (NT), 0, s, gf, g, l, B));
+}
+
+int bmg_blocks_correct (int dim, int odd, bmg_geom g, int l, bmg_blocks B, cudaStream_t s)
+{
+  const dim3 gb = grid_of (1LL << (dim*l), B.m);
+  return status_of (dim == 1 ? pdl_launch (k_blocks_correct<1>, gb, dim3 (NT), 0, s, g, l, B, odd)
+                    : dim == 2 ? pdl_launch (k_blocks_correct<2>, gb, dim3 (NT), 0, s, g, l, B, odd)
+                    : pdl_launch (k_blocks_correct<3>, gb, dim3 (NT), 0, s, g, l, B, odd));
+}
+
+int bmg_blocks_residual (int dim, bmg_geom g, int l, bmg_blocks B, double Delta,
+                         unsigned long long * maxres, cudaStream_t s)
+{
+  const dim3 gb = grid_of (1LL << (dim*l), B.m);
+  auto run = [&] (auto kern) { return pdl_launch (kern, gb, dim3 (NT), 0, s, g, l, B, Delta, maxres); };
+  const bool p2 = delta_pow2 (Delta);
+  return status_of (dim == 1 ? (p2 ? run (k_blocks_residual<1, true>) : run (k_blocks_residual<1, false>))
+                    : dim == 2 ? (p2 ? run (k_blocks_residual<2, true>) : run (k_blocks_residual<2, false>))
+                    : p2 ? run (k_blocks_residual<3, true>) : run (k_blocks_residual<3, false>));
+}
+
+int bmg_blocks_bottom (int dim, const bmg_geom * g, const double * Delta, int lo, int hi,
+                       bmg_blocks B, int nrelax, int restrict_src, cudaStream_t s)
+{
+  if (lo < 1 || hi < lo || hi > BMG_MAXLEVEL) return (int) cudaErrorInvalidValue;
+  BottomParams P;
+  memset (&P, 0, sizeof P);
+  for (int l = lo; l <= hi + (restrict_src ? 1 : 0); l++) { P.g[l] = g[l]; P.Delta[l] = Delta[l]; }
+  P.B = B; P.lo = lo; P.hi = hi; P.nrelax = nrelax; P.restrict_src = restrict_src;
+  return status_of (dim == 1 ? pdl_launch (k_blocks_bottom<1>, dim3 (1), dim3 (1024), 0, s, P)
+                    : dim == 2 ? pdl_launch (k_blocks_bottom<2>, dim3 (1), dim3 (1024), 0, s, P)
+                    : pdl_launch (k_blocks_bottom<3>, dim3 (1), dim3 (1024), 0, s, P));
+}
+
+} // extern "C"

@@ -8,6 +8,7 @@
 #define MG_DEVICE_CUH
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include "mg_launch.h"
 
 namespace bmgd {
@@ -270,6 +271,22 @@ __device__ __forceinline__ T relax_value (const bmg_geom & g, long long id, cons
     d += a1 + a0;
   }
   return nn/d;
+}
+
+/* x/Delta; when Delta is a power of two (L0 = 1, Delta = 2^-l) the
+   division is an exact scaling and x*(1/Delta) is the same double, at a
+   fraction of the cost of the IEEE division */
+template <bool POW2>
+__device__ __forceinline__ double over_delta (double x, double Delta, double rDelta)
+{
+  return POW2 ? x*rDelta : x/Delta;
+}
+
+/* whether x*(1/Delta) is that double */
+inline bool delta_pow2 (double Delta)
+{
+  int ex;
+  return Delta > 0. && frexp (Delta, &ex) == 0.5 && ex > -1000 && ex < 1000;
 }
 
 /* ---------------------------------------------------------------- */

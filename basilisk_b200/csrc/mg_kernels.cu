@@ -331,15 +331,6 @@ __global__ void k_restrict_face (bmg_geom gf, bmg_geom gc, FacePtrs p, int level
 /* residual + max reduction                                          */
 /* ---------------------------------------------------------------- */
 
-/* x/Delta; when Delta is a power of two (L0 = 1, Delta = 2^-l) the
-   division is an exact scaling and x*(1/Delta) is the same double, at a
-   fraction of the cost of the IEEE division */
-template <bool POW2>
-__device__ __forceinline__ double over_delta (double x, double Delta, double rDelta)
-{
-  return POW2 ? x*rDelta : x/Delta;
-}
-
 template <int DIM, typename TR, bool POW2>
 __global__ void k_residual (bmg_geom g, bmg_geom gr, const double * __restrict__ a,
                             const double * __restrict__ b, Coef<double> ax,
@@ -887,8 +878,7 @@ void residual_dim (int st, bmg_geom g, bmg_geom gr, const double * a, const doub
   Coef<double> ax = coef_of<double> (alpha[0]), ay = coef_of<double> (alpha[1]),
     az = coef_of<double> (alpha[2]), lam = coef_of<double> (lambda);
   dim3 gb = grid_shape<DIM> (g.n), bb = block_shape<DIM> ();
-  int ex;
-  const bool pow2 = Delta > 0. && frexp (Delta, &ex) == 0.5 && ex > -1000 && ex < 1000;
+  const bool pow2 = delta_pow2 (Delta);
   if (st == BMG_ST_F64) {
     if (pow2) pdl_launch (k_residual<DIM, double, true>, gb, bb, 0, s, g, gr, a, b, ax, ay, az, lam, Delta, (double *) res, maxres);
     else pdl_launch (k_residual<DIM, double, false>, gb, bb, 0, s, g, gr, a, b, ax, ay, az, lam, Delta, (double *) res, maxres);
@@ -908,8 +898,7 @@ void residual_restrict_2d (bmg_geom g, bmg_geom gr, bmg_geom gc, const double * 
   Coef<double> ax = coef_of<double> (alpha[0]), ay = coef_of<double> (alpha[1]),
     lam = coef_of<double> (lambda);
   const dim3 bb (32, 8, 1), gb ((gc.n + 31)/32, (gc.n + 7)/8, 1);
-  int ex;
-  const bool pow2 = Delta > 0. && frexp (Delta, &ex) == 0.5 && ex > -1000 && ex < 1000;
+  const bool pow2 = delta_pow2 (Delta);
   if (pow2)
     pdl_launch (k_residual_restrict2d<TR, TC, true>, gb, bb, 0, s, g, gr, gc, a, b, ax, ay, lam,
                 Delta, (TR *) res, (TC *) resc, maxres);
@@ -927,8 +916,7 @@ void residual_restrict_3d (bmg_geom g, bmg_geom gr, bmg_geom gc, const double * 
   Coef<double> ax = coef_of<double> (alpha[0]), ay = coef_of<double> (alpha[1]),
     az = coef_of<double> (alpha[2]), lam = coef_of<double> (lambda);
   const dim3 bb = block_shape<3> (), gb = grid_shape<3> (gc.n);
-  int ex;
-  const bool pow2 = Delta > 0. && frexp (Delta, &ex) == 0.5 && ex > -1000 && ex < 1000;
+  const bool pow2 = delta_pow2 (Delta);
   if (pow2)
     pdl_launch (k_residual_restrict3d<TR, TC, true>, gb, bb, 0, s, g, gr, gc, a, b, ax, ay, az,
                 lam, Delta, (TR *) res, (TC *) resc, maxres);

@@ -16,22 +16,24 @@
  *
  * Here every block is a bmg_grid on a CUDA device, and one host thread
  * drives all the blocks of the decomposition: the blocks of one device
- * share one stream, the exchange of a direction is one kernel per device
- * (bmg_launch_halo) that copies every neighbour's edge slab straight into
- * its blocks' ghost slabs -- reading the neighbour by peer access over
- * NVLink when it lives on another device -- ordered across devices by
- * events, and the reductions are the maximum / sum of the blocks' values
- * on the host, which reads them back every cycle as the single-grid solve
- * does.
+ * share one stream and one launch per operation (mg_blocks.cu), in which the
+ * thread that writes a cell also writes its images in the neighbours' ghost
+ * layers -- over NVLink when the neighbour lives on another device -- so
+ * that no exchange follows; operations are ordered across devices by
+ * events.  Only a, as it comes in, has its ghosts exchanged by slabs
+ * (bmg_launch_halo).  The reductions are the maximum / sum of the devices'
+ * values on the host, which reads them back every cycle as the single-grid
+ * solve does.
  *
  * Boundary conditions: a side of a block that faces another block keeps
- * the field's box condition type (its kernels write box images there,
- * which the exchange then overwrites); a direction is periodic on a block
- * only when the domain is periodic in it and it holds a single block.
+ * the field's box condition type, which is not applied there; a direction
+ * is periodic on a block only when the domain is periodic in it and it holds
+ * a single block.
  *
  * The solve is the reference's mg_solve / mg_cycle (poisson.h:32-90,
- * 139-235) with one relaxation pass per launch and a boundary exchange
- * after each pass, exactly where the single-grid solve has a boundary: the
+ * 139-235) with one relaxation pass per launch (the coarse levels in one
+ * launch of one CTA) and the boundary with each pass, exactly where the
+ * single-grid solve has one: the
  * zero or prolonged correction of a level, each colour pass of a red-black
  * sweep (red, boundary, black, boundary) or each Jacobi sweep, and a after
  * the correction a += da.  Every value is computed by the kernels the
@@ -47,6 +49,7 @@
 #include <cuda_runtime_api.h>
 
 #include "mg_grid.h"
+#include "mg_blocks.h"
 
 #define MAXB 4096
 
@@ -61,6 +64,15 @@ struct bmg_shard {
   int * bdev;                 /* device slot of each block */
   bmg_halo * halo;            /* exchange descriptors, one per block */
   long long nhalo;            /* exchange launches */
+  /* the tables of the blocks' kernels (mg_blocks.h): the host's copy, and
+     each device's, written when a solve's differ from the last one's */
+  size_t tbytes;
+  bmg_blk * tblk;
+  bmg_blk_level * tlv;
+  void * dtab[16];
+  int tables;
+  int first[16];              /* the first block of each device */
+  bmg_blocks B[16];
 };
 
 #define FAIL(s) bmg_i_fail (s)
@@ -152,7 +164,9 @@ void bmg_shard_free (bmg_shard * s)
     cudaSetDevice (s->dev[k]);
     if (s->stream[k]) cudaStreamDestroy (s->stream[k]);
     if (s->ev[k]) cudaEventDestroy (s->ev[k]);
+    cudaFree (s->dtab[k]);
   }
+  free (s->tblk);
   free (s->blk); free (s->nbr); free (s->bdev); free (s->halo);
   free (s);
 }
@@ -308,12 +322,6 @@ static double * ptr_a (bmg_shard * s, int b, int l, void * data)
   return ((blk_t *) data)[b].a->lv[l];
 }
 
-static double * ptr_da (bmg_shard * s, int b, int l, void * data)
-{
-  (void) data;
-  return bmg_i_ws64 (s->blk[b], BMG_WS_DA, l);
-}
-
 static double delta_of (const bmg_grid * g, int l) { return g->L0*(1./(1 << l)); }
 
 static int level0_periodic (const bmg_grid * g, int l)
@@ -369,30 +377,95 @@ static int block_coefs (bmg_grid * g, const struct Poisson * p, blk_t * k)
   return BMG_OK;
 }
 
-/* the residual of every block (after the exchange of a), each block's
-   maximum into its pinned host word; with done, an event on block 0's
-   stream after every device's residual */
-static int residual_issue (bmg_shard * s, blk_t * k, cudaEvent_t done)
+/* the tables of the blocks' kernels for this solve, on every device:
+   blocks, then levels, then each device's own block indices */
+static int upload_tables (bmg_shard * s, const blk_t * k)
+{
+  const int nb = s->nb, L = s->blk[0]->depth;
+  const size_t nlv = (size_t) (L + 1)*nb;
+  const size_t olv = nb*sizeof (bmg_blk), omine = olv + nlv*sizeof (bmg_blk_level);
+  const size_t bytes = omine + nb*sizeof (int);
+  if (!s->tblk) {
+    if (!(s->tblk = calloc (2, bytes))) return FAIL (BMG_ENOMEM);
+    s->tbytes = bytes;
+    for (int d = 0; d < s->ndev; d++) {
+      CKS (cudaSetDevice (s->dev[d]));
+      CKS (cudaMalloc (&s->dtab[d], bytes));
+    }
+  }
+  /* the second half of the host buffer takes this solve's tables */
+  char * cur = (char *) s->tblk, * now = cur + bytes;
+  memset (now, 0, bytes);
+  bmg_blk * tb = (bmg_blk *) now;
+  s->tlv = (bmg_blk_level *) (now + olv);
+  for (int b = 0; b < nb; b++) {
+    memcpy (tb[b].nbr, s->nbr[b], sizeof tb[b].nbr);
+    tb[b].bc = k[b].abc;
+    tb[b].a = k[b].a->lv[L];
+    tb[b].b = k[b].b->lv[L];
+    for (int l = 0; l <= L; l++) {
+      bmg_blk_level * q = &s->tlv[(size_t) l*nb + b];
+      q->da = bmg_i_ws64 (s->blk[b], BMG_WS_DA, l);
+      q->da2 = bmg_i_ws64 (s->blk[b], BMG_WS_DA2, l);
+      q->res = bmg_i_ws64 (s->blk[b], BMG_WS_RES, l);
+      for (int d = 0; d < 3; d++) q->alpha[d] = k[b].alpha[l][d];
+      q->lambda = k[b].lambda[l];
+    }
+  }
+  int * mine = (int *) (now + omine), m = 0;
+  for (int d = 0; d < s->ndev; d++) {
+    bmg_blocks * B = &s->B[d];
+    const int first = m;
+    s->first[d] = -1;
+    for (int b = 0; b < nb; b++)
+      if (s->bdev[b] == d) {
+        if (s->first[d] < 0) s->first[d] = b;
+        mine[m++] = b;
+      }
+    B->blk = (const bmg_blk *) s->dtab[d];
+    B->lv = (const bmg_blk_level *) ((char *) s->dtab[d] + olv);
+    B->mine = (const int *) ((char *) s->dtab[d] + omine) + first;
+    B->nb = nb; B->m = m - first;
+  }
+  if (!s->tables || memcmp (cur, now, bytes)) {
+    s->tables = 0;
+    for (int d = 0; d < s->ndev; d++) {
+      CKS (cudaSetDevice (s->dev[d]));
+      CKS (cudaMemcpyAsync (s->dtab[d], now, bytes, cudaMemcpyHostToDevice, s->stream[d]));
+    }
+    for (int d = 0; d < s->ndev; d++) CKS (cudaStreamSynchronize (s->stream[d]));
+    memcpy (cur, now, bytes);
+    s->tables = 1;
+  }
+  return BMG_OK;
+}
+
+/* one operation on every device (d: its slot, B: its blocks), complete on
+   all of them before the next starts on any */
+#define EACH(call) do { for (int d = 0; d < s->ndev; d++) { \
+      const bmg_blocks B = s->B[d]; \
+      CKS (cudaSetDevice (s->dev[d])); \
+      CLS (call); } \
+    int r_ = sync_devices (s); if (r_) return r_; } while (0)
+
+/* the residual of every block, the ghosts of a in place, each device's
+   maximum into the pinned word of its first block; with done, an event on
+   block 0's stream after every device's residual */
+static int residual_issue (bmg_shard * s, cudaEvent_t done)
 {
   const int L = s->blk[0]->depth;
-  int r = exchange (s, L, ptr_a, k);
-  if (r) return r;
-  for (int b = 0; b < s->nb; b++) {
-    bmg_grid * g = s->blk[b];
-    CKS (cudaSetDevice (g->device));
-    CKS (cudaMemsetAsync (g->d_maxres, 0, sizeof (unsigned long long), g->stream));
-    CLS (bmg_launch_residual (g->dim, BMG_ST_F64, g->g64[L], g->g64[L], k[b].a->lv[L],
-                              k[b].b->lv[L], k[b].alpha[L], k[b].lambda[L], delta_of (g, L),
-                              bmg_i_ws64 (g, BMG_WS_RES, L), g->d_maxres, g->stream));
+  for (int d = 0; d < s->ndev; d++) {
+    CKS (cudaSetDevice (s->dev[d]));
+    CKS (cudaMemsetAsync (s->blk[s->first[d]]->d_maxres, 0, sizeof (unsigned long long), s->stream[d]));
   }
+  EACH (bmg_blocks_residual (s->dim, s->blk[0]->g64[L], L, B, delta_of (s->blk[0], L),
+                             s->blk[s->first[d]]->d_maxres, s->stream[d]));
   if (done) {
-    int r2 = sync_devices (s);
-    if (r2) return r2;
     CKS (cudaSetDevice (s->blk[0]->device));
     CKS (cudaEventRecord (done, s->blk[0]->stream));
   }
-  for (int b = 0; b < s->nb; b++) {
-    bmg_grid * g = s->blk[b];
+  for (int d = 0; d < s->ndev; d++) {
+    bmg_grid * g = s->blk[s->first[d]];
     CKS (cudaSetDevice (g->device));
     CKS (cudaMemcpyAsync (g->h_pinned, g->d_maxres, sizeof (double),
                           cudaMemcpyDeviceToHost, g->stream));
@@ -400,13 +473,13 @@ static int residual_issue (bmg_shard * s, blk_t * k, cudaEvent_t done)
   return BMG_OK;
 }
 
-/* max over the blocks of their residual maxima (non-negative doubles, or
+/* max over the devices of their residual maxima (non-negative doubles, or
    NaN, compared by their bits as the kernels' atomicMax does) */
 static int residual_collect (bmg_shard * s, double * maxres)
 {
   unsigned long long m = 0;
-  for (int b = 0; b < s->nb; b++) {
-    bmg_grid * g = s->blk[b];
+  for (int d = 0; d < s->ndev; d++) {
+    bmg_grid * g = s->blk[s->first[d]];
     CKS (cudaSetDevice (g->device));
     CKS (cudaStreamSynchronize (g->stream));
     unsigned long long v;
@@ -417,14 +490,12 @@ static int residual_collect (bmg_shard * s, double * maxres)
   return BMG_OK;
 }
 
-static int residual_all (bmg_shard * s, blk_t * k, double * maxres, cudaEvent_t done)
+static int residual_all (bmg_shard * s, double * maxres, cudaEvent_t done)
 {
-  int r = residual_issue (s, k, done);
+  int r = residual_issue (s, done);
   return r ? r : residual_collect (s, maxres);
 }
 
-/* mg_cycle (poisson.h:32-90) over the blocks, one pass per launch, with
-   the boundary exchanges of the single-grid cycle */
 static long long cells_of (int dim, int l)
 {
   long long c = 1;
@@ -450,74 +521,82 @@ static double cycle_bytes (const bmg_shard * s, const blk_t * k, int nrelax, int
   return b*s->nb;
 }
 
-static int shard_cycle (bmg_shard * s, blk_t * k, int nrelax, int minlevel, int maxlevel,
-                        long long * launches)
+/* a red-black sweep of blocks of one cell: the cells of neighbouring blocks
+   read one another in the same pass, so each pass is a launch per block on
+   the ghosts of the pass before, and then the exchange */
+static double * ptr_da0 (bmg_shard * s, int b, int l, void * data)
 {
-  const int dim = s->dim, L = s->blk[0]->depth;
-  const int jacobi = s->blk[0]->relax == BMG_RELAX_JACOBI;
-  /* restriction (res) (multigrid-common.h:368-404): interior cells only */
-  for (int b = 0; b < s->nb; b++) {
-    bmg_grid * g = s->blk[b];
-    CKS (cudaSetDevice (g->device));
-    for (int l = L - 1; l >= minlevel; l--) {
-      CLS (bmg_launch_restrict (dim, BMG_ST_F64, BMG_ST_F64, g->g64[l + 1], g->g64[l],
-                                bmg_i_ws64 (g, BMG_WS_RES, l + 1), bmg_i_ws64 (g, BMG_WS_RES, l),
-                                g->stream));
-      (*launches)++;
-    }
-  }
-  for (int l = minlevel; l <= maxlevel; l++) {
+  (void) data;
+  return bmg_i_ws64 (s->blk[b], BMG_WS_DA, l);
+}
+
+static int single_cell_sweep (bmg_shard * s, blk_t * k, long long * launches)
+{
+  for (int c = 0; c < 2; c++) {
     for (int b = 0; b < s->nb; b++) {
       bmg_grid * g = s->blk[b];
       CKS (cudaSetDevice (g->device));
-      double * da = bmg_i_ws64 (g, BMG_WS_DA, l);
-      if (l == minlevel)
-        CLS (bmg_launch_prolong (dim, BMG_ST_F64, BMG_ST_F64, g->g64[l], g->g64[l], NULL, da,
-                                 &k[b].dabc, 1, g->stream));
-      else
-        CLS (bmg_launch_prolong (dim, BMG_ST_F64, BMG_ST_F64, g->g64[l - 1], g->g64[l],
-                                 bmg_i_ws64 (g, BMG_WS_DA, l - 1), da, &k[b].dabc, 0, g->stream));
+      double * da = bmg_i_ws64 (g, BMG_WS_DA, 0);
+      CLS (bmg_launch_relax (s->dim, BMG_ST_F64, c ? BMG_SWEEP_BLACK : BMG_SWEEP_RED, g->g64[0], da,
+                             da, bmg_i_ws64 (g, BMG_WS_RES, 0), k[b].alpha[0], k[b].lambda[0],
+                             delta_of (g, 0), &k[b].dabc, g->stream));
       (*launches)++;
     }
-    int r = exchange (s, l, ptr_da, k);
+    int r = exchange (s, 0, ptr_da0, k);
     if (r) return r;
+  }
+  return BMG_OK;
+}
+
+/* mg_cycle (poisson.h:32-90) over the blocks, one pass per launch with its
+   boundary */
+static int shard_cycle (bmg_shard * s, blk_t * k, int nrelax, int minlevel, int maxlevel,
+                        long long * launches)
+{
+  const int dim = s->dim, L = s->blk[0]->depth, nd = s->ndev;
+  const int jacobi = s->blk[0]->relax == BMG_RELAX_JACOBI;
+  const bmg_geom * g = s->blk[0]->g64;
+  double Delta[BMG_MAXLEVEL + 1];
+  for (int l = 0; l <= L; l++) Delta[l] = delta_of (s->blk[0], l);
+  /* the coarse levels of a decomposition on one device: one CTA */
+  int top = minlevel - 1;
+  if (nd == 1 && !jacobi && minlevel >= 1)
+    while (top < maxlevel && cells_of (dim, top + 1)*s->nb <= BMG_BLOCKS_CTA_CELLS) top++;
+  /* restriction (res) (multigrid-common.h:368-404): interior cells only */
+  for (int l = L - 1; l > top && l >= minlevel; l--) {
+    EACH (bmg_blocks_restrict (dim, g[l + 1], g[l], l, B, s->stream[d]));
+    *launches += nd;
+  }
+  int odd = 0;                        /* the iterate of the level below is in da2 */
+  if (top >= minlevel) {
+    EACH (bmg_blocks_bottom (dim, g, Delta, minlevel, top, B, nrelax, top < L, s->stream[d]));
+    (*launches)++;
+  }
+  const bmg_geom none = {0};
+  for (int l = top + 1; l <= maxlevel; l++) {
+    EACH (bmg_blocks_prolong (dim, odd, l == minlevel ? none : g[l - 1], g[l], l, B, s->stream[d]));
+    *launches += nd;
+    odd = 0;
     for (int i = 0; i < nrelax; i++) {
-      const int passes = jacobi ? 1 : 2;
-      for (int c = 0; c < passes; c++) {
-        for (int b = 0; b < s->nb; b++) {
-          bmg_grid * g = s->blk[b];
-          CKS (cudaSetDevice (g->device));
-          double * da = bmg_i_ws64 (g, BMG_WS_DA, l);
-          double * res = bmg_i_ws64 (g, BMG_WS_RES, l);
-          if (jacobi) {
-            /* out = (da + 2 n/d)/3 into the partner, then copied back so
-               that da stays the current iterate */
-            double * da2 = bmg_i_ws64 (g, BMG_WS_DA2, l);
-            CLS (bmg_launch_relax (dim, BMG_ST_F64, BMG_SWEEP_JACOBI, g->g64[l], da2, da, res,
-                                   k[b].alpha[l], k[b].lambda[l], delta_of (g, l), &k[b].dabc,
-                                   g->stream));
-            CKS (cudaMemcpyAsync (da, da2, g->g64[l].size*sizeof (double),
-                                  cudaMemcpyDeviceToDevice, g->stream));
-          }
-          else
-            CLS (bmg_launch_relax (dim, BMG_ST_F64, c ? BMG_SWEEP_BLACK : BMG_SWEEP_RED,
-                                   g->g64[l], da, da, res, k[b].alpha[l], k[b].lambda[l],
-                                   delta_of (g, l), &k[b].dabc, g->stream));
-          (*launches)++;
-        }
-        r = exchange (s, l, ptr_da, k);
+      if (jacobi) {
+        EACH (bmg_blocks_relax (dim, BMG_SWEEP_JACOBI, odd, g[l], l, B, Delta[l], s->stream[d]));
+        odd ^= 1;
+        *launches += nd;
+      }
+      else if (l == 0) {
+        int r = single_cell_sweep (s, k, launches);
         if (r) return r;
+      }
+      else {
+        EACH (bmg_blocks_relax (dim, BMG_SWEEP_RED, 0, g[l], l, B, Delta[l], s->stream[d]));
+        EACH (bmg_blocks_relax (dim, BMG_SWEEP_BLACK, 0, g[l], l, B, Delta[l], s->stream[d]));
+        *launches += 2*nd;
       }
     }
   }
   /* a += da with the boundary conditions of a (poisson.h:84-89) */
-  for (int b = 0; b < s->nb; b++) {
-    bmg_grid * g = s->blk[b];
-    CKS (cudaSetDevice (g->device));
-    CLS (bmg_launch_correct (dim, BMG_ST_F64, g->g64[L], g->g64[L], k[b].a->lv[L],
-                             bmg_i_ws64 (g, BMG_WS_DA, L), &k[b].abc, g->stream));
-    (*launches)++;
-  }
+  EACH (bmg_blocks_correct (dim, odd, g[L], L, B, s->stream[d]));
+  *launches += nd;
   return BMG_OK;
 }
 
@@ -564,12 +643,21 @@ int bmg_shard_poisson (bmg_shard * s, struct Poisson p, mgstats * out)
     if (!r && cudaMemcpyAsync (g->h_pinned + 1, g->d_sum, sizeof (double),
                                cudaMemcpyDeviceToHost, g->stream) != cudaSuccess)
       r = BMG_ECUDA;
-    if (!r && cudaStreamSynchronize (g->stream) != cudaSuccess) r = BMG_ECUDA;
-    if (!r) st.sum += g->h_pinned[1];
   }
   if (r) { free (k); cudaSetDevice (cur); return FAIL (BMG_ECUDA); }
   st.nrelax = p.nrelax > 0 ? p.nrelax : 4;
-  r = residual_all (s, k, &st.resb, NULL);
+  r = upload_tables (s, k);
+  /* the ghosts of a as it comes in (the corrections write them afterwards) */
+  if (!r) r = exchange (s, L, ptr_a, k);
+  if (!r) r = residual_all (s, &st.resb, NULL);
+  if (!r) for (int b = 0; b < s->nb; b++) {
+    bmg_grid * g = s->blk[b];
+    if (cudaSetDevice (g->device) != cudaSuccess || cudaStreamSynchronize (g->stream) != cudaSuccess) {
+      r = FAIL (BMG_ECUDA);
+      break;
+    }
+    st.sum += g->h_pinned[1];
+  }
   double resb = st.resa = st.resb;
   int status = BMG_OK;
   bmg_grid * g0 = s->blk[0];
@@ -583,7 +671,7 @@ int bmg_shard_poisson (bmg_shard * s, struct Poisson p, mgstats * out)
     }
     const double bytes = cycle_bytes (s, k, st.nrelax, minlevel, L);
     if (!r) r = shard_cycle (s, k, st.nrelax, minlevel, L, &launches);
-    if (!r) r = residual_all (s, k, &st.resa, g0->timing ? g0->ev1 : NULL);
+    if (!r) r = residual_all (s, &st.resa, g0->timing ? g0->ev1 : NULL);
     if (r) break;
     g0->counters.cycles++;
     g0->counters.bytes += bytes;

@@ -129,3 +129,43 @@ def test_two_blocks_rectangular_domain():
     sg.close()
     np.testing.assert_array_equal(sol[:n], sol[n:])
 
+
+@pytest.mark.parametrize("relax", ["rbgs", "jacobi"])
+@pytest.mark.parametrize("dim,depth,dims,periodic", [(1, 3, (4,), False), (2, 2, (2, 2), False),
+                                                     (2, 3, (4, 4), True), (2, 6, (2, 2), True),
+                                                     (2, 7, (2, 2), False), (2, 8, (4, 4), False),
+                                                     (3, 2, (2, 2, 2), False), (3, 3, (4, 4, 4), True),
+                                                     (3, 5, (2, 2, 2), False)])
+def test_blocks_around_the_single_cta_levels_bit_identical(dim, depth, dims, periodic, relax):
+    """Blocks of two cells and up, whose levels lie below, at and above the
+    cells that one CTA relaxes for all blocks (all their images -- edges and
+    corners, box, periodic and neighbouring -- written by the owners)."""
+    import helpers
+    rng = np.random.default_rng(100 * dim + depth)
+    kinds = [("dirichlet", 0.5), ("neumann", -0.25), ("dirichlet", -1.0), ("neumann", 0.75),
+             ("neumann", 0.5), ("dirichlet", 0.25)]
+    if periodic:
+        prob = helpers.random_problem(dim, depth, rng, periodic=tuple(range(dim)), lam="field")
+        for d, c in enumerate(prob["alpha"]):    # face n of a periodic direction is face 0
+            c[(slice(None),) * d + (-1,)] = c[(slice(None),) * d + (0,)]
+    else:
+        prob = helpers.random_problem(dim, depth, rng, bc={s: kinds[s] for s in range(2 * dim)}, lam="field")
+    compare(prob, dims, relax, 1e-8)
+
+
+def test_blocks_of_one_cell():
+    """2 x 2 blocks of a single cell, Dirichlet 0, alpha = 1: the solution of
+    the 4 x 4 system (each cell: -6 a + two neighbours = b Delta^2).  Every
+    cell relaxes from the last pass's neighbours and ghosts, which leaves the
+    chequered mode undamped: b has none of it."""
+    sg = ShardedGrid(2, 0, dims=(2, 2), relax="rbgs")
+    a = sg.scalar()
+    for side in ("right", "left", "top", "bottom"):
+        a.bc(side, "dirichlet", 0.0)
+    b = np.array([[6.0, 0.0], [2.0, -4.0]])
+    a.set(np.zeros((2, 2)))
+    st = sg.poisson(a, sg.scalar(b), tolerance=1e-9)
+    assert st["status"] == 0 and st["resa"] <= 1e-9, st
+    A = np.array([[-6, 1, 1, 0], [1, -6, 0, 1], [1, 0, -6, 1], [0, 1, 1, -6]], float)
+    np.testing.assert_allclose(a.get().ravel(), np.linalg.solve(A, b.ravel() / 4.0), atol=1e-10)
+    sg.close()
