@@ -460,6 +460,19 @@ __device__ __forceinline__ void field_op (const bmg_tree_op & op, long gt, long 
     }
     break;
   }
+  case BMG_TI_CELLS: {
+    const long w = op.n + op.sub;
+    for (long k = gt; k < w + op.nr; k += gs) {
+      if (k >= w) ghost_value<ICG> (op.rules[k - w], T, s, bc, op.homog);
+      else if (k >= op.n) {
+        int l, i, j;
+        unpack (list[k], l, i, j);
+        s[gidx (T, l, i, j)] = bilinear<ICG> (T, s, l, i, j);
+      }
+      else restrict_cell<ICG> (list, k, T, s);
+    }
+    break;
+  }
   }
 #undef ENTRY
 }
@@ -533,6 +546,7 @@ k_tree_interp (const bmg_tree_op * __restrict__ ops, int nops, TL Tp, double * f
     case BMG_TI_PROLONG:
     case BMG_TI_RESTRICT:
     case BMG_TI_STAGE:
+    case BMG_TI_CELLS:
       if (op.field == 0) field_op (op, g0, gsx, first, T, fa, B[op.bcsel]);
       else field_op (op, g0, gsx, first, T, F[op.field], B[op.bcsel]);
       break;

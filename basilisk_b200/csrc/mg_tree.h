@@ -105,12 +105,14 @@ int bmg_tree_launch_add (const uint32_t * leaves, long n, const bmg_tree_levels 
    (0 a, 1 da, 2 res, 3 the Jacobi temporary), the boundary conditions of a
    ghost rule (bcsel: 0 those of a, 1 those of da) and whether they are
    homogeneous; sub is a stage's operation, or for a relaxation 1 when it
-   writes the Jacobi temporary; v is the value of a set; local marks an
+   writes the Jacobi temporary; BMG_TI_CELLS computes single cells: list
+   holds n refined cells to restrict, then sub halo cells to prolong, and
+   rules nr ghosts; v is the value of a set; local marks an
    operation small enough for one CTA (the interpreter runs it on the
    cluster's first CTA alone and separates two consecutive local
    operations by a CTA barrier instead of a cluster barrier) */
 enum { BMG_TI_SET = 0, BMG_TI_PROLONG, BMG_TI_RESTRICT, BMG_TI_STAGE, BMG_TI_RELAX,
-       BMG_TI_JACOBI, BMG_TI_ADD, BMG_TI_RESIDUAL };
+       BMG_TI_JACOBI, BMG_TI_ADD, BMG_TI_RESIDUAL, BMG_TI_CELLS };
 typedef struct {
   const uint32_t * list;
   long long n;

@@ -47,6 +47,10 @@ typedef struct { long off, n; } span_t;
 typedef struct { int op; span_t list; span_t rules; } tstage;
 enum { SCHED_FULL = 0, SCHED_PRUNED = 1 };
 
+/* one stage of the correction's boundary by dependence (depend ()): refined
+   cells, halo cells and ghosts whose sources earlier stages computed */
+typedef struct { long off, nrest, nhalo; span_t rules; } tdep;
+
 /* everything a captured solve iteration depends on */
 typedef struct {
   int nrelax, minlevel, maxlevel, relax, mixed;
@@ -85,6 +89,12 @@ struct bmg_tree {
   long nstages;
   span_t sched[2][TMAX + 1];
   bmg_tree_rule * dsrules;
+  /* the correction's boundary of each level by dependence: spans of deps,
+     whose cells and rules live in ddlist and ddrules */
+  tdep * deps;
+  span_t dep[TMAX + 1];
+  uint32_t * ddlist;
+  bmg_tree_rule * ddrules;
   bmg_tree_levels T;
   double * dpart;
   int npart;
@@ -131,8 +141,8 @@ static void tree_release (struct bmg_tree * t)
   for (int i = 0; i < NTGRAPH; i++) graph_drop (&t->graphs[i]);
   for (int l = 0; l <= TMAX; l++) { free (t->fl[l]); free (t->nb[l]); }
   cudaFree (t->dflags); cudaFree (t->dlist); cudaFree (t->drules); cudaFree (t->dpart);
-  cudaFree (t->dsrules); cudaFree (t->ws32);
-  free (t->stages);
+  cudaFree (t->dsrules); cudaFree (t->ws32); cudaFree (t->ddlist); cudaFree (t->ddrules);
+  free (t->stages); free (t->deps);
   free (t);
 }
 
@@ -351,6 +361,162 @@ static int schedule (struct bmg_tree * t, int l, int mlo, const bmg_tree_rule * 
   return BMG_OK;
 }
 
+/* The boundary of the correction by dependence.  A pass of relax on level l
+   reads the neighbours of its set (the active cells of level l and the
+   leaves below), and the prolongation to level l + 1 the 3 x 3
+   neighbourhoods of level l: of the cells that tree_boundary_level computes
+   only those outside the set that one of these reads, and their sources
+   among each other, matter.  Each such cell -- restricted (refined), halo
+   (prolonged) or ghost -- goes into the stage after the last of its sources:
+   two stages on the band trees (a restricted cell at a refinement edge has
+   leaf children, a halo cell reads those and leaves), where the restriction
+   and prolongation of every level took up to two per level (438 -> 284 ms per
+   solve of the depth-10 band tree).  The values are those of the full
+   sequence: the same expressions on the same sources. */
+typedef struct {
+  struct bmg_tree * t;
+  int l, err;
+  unsigned char * mark[TMAX + 1];    /* 0: not visited, else stage + 1 */
+  uint32_t * cell;                   /* the visited cells, and their stages */
+  long n, cap;
+} depset;
+
+static int dep_inset (const depset * s, int m, int i, int j)
+{
+  const int n = 1 << m;
+  if (i < 0 || j < 0 || i >= n || j >= n) return 0;
+  const unsigned char f = s->t->fl[m][HX (m, i, j)];
+  return (f & BMG_T_ACTIVE) && (m == s->l || (f & BMG_T_LEAF));
+}
+
+/* the stage of a cell: 0 in the set (or never computed), else after its
+   sources */
+static int dep_visit (depset * s, int m, int i, int j)
+{
+  if (dep_inset (s, m, i, j)) return 0;
+  unsigned char * mk = &s->mark[m][HX (m, i, j)];
+  if (*mk) return *mk - 1;
+  const int n = 1 << m;
+  int d = 0;
+#define SRC(m_, i_, j_) do { const int q_ = dep_visit (s, m_, i_, j_); if (q_ > d) d = q_; } while (0)
+  if (i < 0 || j < 0 || i >= n || j >= n) {
+    bmg_tree_rule r;
+    if (!ghost_rule (s->t, m, i, j, &r)) { *mk = 1; return 0; }
+    SRC (m, (int) ((r.inner >> 14) & 0x3FFF) - 1, (int) (r.inner & 0x3FFF) - 1);
+  }
+  else {
+    const unsigned char f = s->t->fl[m][HX (m, i, j)];
+    if (f & BMG_T_ACTIVE) {
+      for (int c = 0; c < 4; c++) SRC (m + 1, 2*i + (c >> 1), 2*j + (c & 1));
+    }
+    else if ((f & BMG_T_HALO) && m > 0) {
+      const int pi = i >> 1, pj = j >> 1, cx = (i & 1) ? 1 : -1, cy = (j & 1) ? 1 : -1;
+      SRC (m - 1, pi, pj); SRC (m - 1, pi + cx, pj); SRC (m - 1, pi, pj + cy); SRC (m - 1, pi + cx, pj + cy);
+    }
+    else { *mk = 1; return 0; }
+  }
+#undef SRC
+  d++;
+  *mk = (unsigned char) (d + 1);
+  if (s->n == s->cap) {
+    const long cap = 2*s->cap + 1024;
+    uint32_t * c = realloc (s->cell, cap*sizeof (uint32_t));
+    if (!c) { s->err = 1; return d; }
+    s->cell = c; s->cap = cap;
+  }
+  s->cell[s->n++] = pack (m, i, j);
+  return d;
+}
+
+/* the stages of every level, uploaded; h: the host cell lists */
+static int depend (struct bmg_tree * t, const uint32_t * h)
+{
+  depset s;
+  memset (&s, 0, sizeof s);
+  s.t = t;
+  uint32_t * list = NULL;
+  bmg_tree_rule * rules = NULL;
+  long nlist = 0, nrules = 0, caplist = 0, caprules = 0, ndeps = 0, capdeps = 0;
+  free (t->deps); t->deps = NULL;
+  for (int l = 0; l <= t->depth && !s.err; l++) {
+    const size_t m = (size_t) ((1 << l) + 2)*((1 << l) + 2);
+    if (!(s.mark[l] = malloc (m))) s.err = 1;
+  }
+  for (int l = 0; l <= t->depth && !s.err; l++) {
+    s.l = l; s.n = 0;
+    for (int m = 0; m <= l; m++) memset (s.mark[m], 0, (size_t) ((1 << m) + 2)*((1 << m) + 2));
+    for (long k = 0; k < t->rl[l].n; k++) {
+      const uint32_t e = h[t->rl[l].off + k];
+      const int m = (int) (e >> 28), i = (int) ((e >> 14) & 0x3FFF) - 1, j = (int) (e & 0x3FFF) - 1;
+      dep_visit (&s, m, i - 1, j); dep_visit (&s, m, i + 1, j);
+      dep_visit (&s, m, i, j - 1); dep_visit (&s, m, i, j + 1);
+    }
+    /* the neighbourhoods of the refined cells of level l */
+    for (long k = 0; k < t->ref[l].n; k++) {
+      const uint32_t e = h[t->ref[l].off + k];
+      const int i = (int) ((e >> 14) & 0x3FFF) - 1, j = (int) (e & 0x3FFF) - 1;
+      for (int a = -1; a <= 1; a++)
+        for (int b = -1; b <= 1; b++) dep_visit (&s, l, i + a, j + b);
+    }
+    int last = 0;
+    for (long k = 0; k < s.n; k++) {
+      const uint32_t e = s.cell[k];
+      const int m = (int) (e >> 28);
+      const int d = s.mark[m][HX (m, (int) ((e >> 14) & 0x3FFF) - 1, (int) (e & 0x3FFF) - 1)] - 1;
+      if (d > last) last = d;
+    }
+    t->dep[l].off = ndeps; t->dep[l].n = last;
+    if (ndeps + last > capdeps) {
+      capdeps = 2*capdeps + last;
+      tdep * q = realloc (t->deps, capdeps*sizeof (tdep));
+      if (!q) { s.err = 1; break; }
+      t->deps = q;
+    }
+    if (nlist + s.n > caplist) {
+      caplist = 2*caplist + s.n;
+      uint32_t * q = realloc (list, caplist*sizeof (uint32_t));
+      if (!q) { s.err = 1; break; }
+      list = q;
+    }
+    if (nrules + s.n > caprules) {
+      caprules = 2*caprules + s.n;
+      bmg_tree_rule * q = realloc (rules, caprules*sizeof (bmg_tree_rule));
+      if (!q) { s.err = 1; break; }
+      rules = q;
+    }
+    for (int d = 1; d <= last; d++) {
+      tdep * st = &t->deps[ndeps++];
+      st->off = nlist; st->nrest = st->nhalo = 0;
+      st->rules.off = nrules; st->rules.n = 0;
+      /* restricted cells, then halo cells, then ghosts */
+      for (int kind = 0; kind < 3; kind++)
+        for (long k = 0; k < s.n; k++) {
+          const uint32_t e = s.cell[k];
+          const int m = (int) (e >> 28), i = (int) ((e >> 14) & 0x3FFF) - 1, j = (int) (e & 0x3FFF) - 1;
+          if (s.mark[m][HX (m, i, j)] - 1 != d) continue;
+          const int n = 1 << m, ghost = i < 0 || j < 0 || i >= n || j >= n;
+          const int ck = ghost ? 2 : (t->fl[m][HX (m, i, j)] & BMG_T_ACTIVE) ? 0 : 1;
+          if (ck != kind) continue;
+          if (kind == 2) { if (ghost_rule (t, m, i, j, &rules[nrules])) { nrules++; st->rules.n++; } }
+          else { list[nlist++] = e; if (kind == 0) st->nrest++; else st->nhalo++; }
+        }
+    }
+  }
+  for (int l = 0; l <= t->depth; l++) free (s.mark[l]);
+  free (s.cell);
+  cudaFree (t->ddlist); cudaFree (t->ddrules);
+  t->ddlist = NULL; t->ddrules = NULL;
+  if (!s.err &&
+      (cudaMalloc ((void **) &t->ddlist, (nlist + 1)*sizeof (uint32_t)) != cudaSuccess ||
+       cudaMalloc ((void **) &t->ddrules, (nrules + 1)*sizeof (bmg_tree_rule)) != cudaSuccess ||
+       (nlist && cudaMemcpy (t->ddlist, list, nlist*sizeof (uint32_t), cudaMemcpyHostToDevice) != cudaSuccess) ||
+       (nrules && cudaMemcpy (t->ddrules, rules, nrules*sizeof (bmg_tree_rule), cudaMemcpyHostToDevice)
+        != cudaSuccess)))
+    s.err = 1;
+  free (list); free (rules);
+  return s.err ? BMG_ENOMEM : BMG_OK;
+}
+
 /* flags of halo cells and prolongation leaves, cell lists, ghost rules:
    the caches of update_cache_f (tree.h:556-684), uploaded */
 static int derive (bmg_grid * g, struct bmg_tree * t)
@@ -468,6 +634,7 @@ static int derive (bmg_grid * g, struct bmg_tree * t)
       cudaMemcpy (t->dlist, h, total*sizeof (uint32_t), cudaMemcpyHostToDevice) != cudaSuccess ||
       (k && cudaMemcpy (t->drules, hr, k*sizeof (bmg_tree_rule), cudaMemcpyHostToDevice) != cudaSuccess))
     st = BMG_ENOMEM;
+  if (!st) st = depend (t, h);
   free (h); free (hf);
   if (st) { free (hr); return FAIL (st); }
   /* boundary schedules */
@@ -685,8 +852,9 @@ static int t_residual (bmg_grid * g, struct bmg_tree * t, double * a, const doub
 /* the iteration as interpreter operations                             */
 /* ------------------------------------------------------------------ */
 
-/* the same operations, in the same order, as the launches of t_cycle and
-   t_residual (an empty operation, which those skip, is left out) */
+/* the operations of t_cycle and t_residual in their order (an empty one,
+   which those skip, is left out), with the correction's boundary by
+   dependence */
 typedef struct {
   bmg_tree_op * v; long n, cap; int err; double bytes; int astored, lstored;
   double vb;            /* bytes of a value of the cycle's fields: 8, or 4 (mixed form) */
@@ -709,6 +877,7 @@ static double item_bytes (const opvec * o, int type, int sub, int rule, int fiel
   case BMG_TI_PROLONG: return 4. + 4*w + w;
   case BMG_TI_RESTRICT: return 4. + 4*w + w;
   case BMG_TI_STAGE: return sub == BMG_T_OP_HALO ? 1. + 4*w + w : 4. + 4*w + w;
+  case BMG_TI_CELLS: return 4. + 4*w + w;
   case BMG_TI_RELAX: return 4. + w + 4*w + 4*ax + lam + w;
   case BMG_TI_JACOBI: return 4. + 2*w + w;
   case BMG_TI_ADD: return 4. + 2*8. + o->vb;
@@ -727,7 +896,8 @@ static void r_push (opvec * o, int type, int field, int sub, int homog, const ui
     if (!nv) { o->err = 1; return; }
     o->v = nv; o->cap = cap;
   }
-  const long items = type == BMG_TI_STAGE ? (sub == BMG_T_OP_HALO ? 4*n : sub == BMG_T_OP_RESTRICT ? n : 0) : n;
+  const long items = type == BMG_TI_STAGE ? (sub == BMG_T_OP_HALO ? 4*n : sub == BMG_T_OP_RESTRICT ? n : 0)
+    : type == BMG_TI_CELLS ? n + sub : n;
   o->bytes += items*item_bytes (o, type, sub, 0, field) + nr*item_bytes (o, type, sub, 1, field);
   bmg_tree_op * q = &o->v[o->n++];
   memset (q, 0, sizeof *q);
@@ -739,6 +909,7 @@ static void r_push (opvec * o, int type, int field, int sub, int homog, const ui
   q->local = items + nr <= 2048;
 }
 
+/* the full boundary of a field (a's, which its user may read) */
 static void r_boundary (struct bmg_tree * t, opvec * o, int field, int l, int homog, int kind)
 {
   if (t->full) {
@@ -758,6 +929,17 @@ static void r_boundary (struct bmg_tree * t, opvec * o, int field, int l, int ho
   }
 }
 
+/* the boundary of da that a pass on level l reads, by dependence */
+static void r_depend (struct bmg_tree * t, opvec * o, int l)
+{
+  for (long k = 0; k < t->dep[l].n; k++) {
+    const tdep * d = &t->deps[t->dep[l].off + k];
+    if (d->nrest + d->nhalo + d->rules.n > 0)
+      r_push (o, BMG_TI_CELLS, F_DA, (int) d->nhalo, 1, t->ddlist + d->off, d->nrest,
+              t->ddrules + d->rules.off, d->rules.n, 0.);
+  }
+}
+
 static void r_relax (bmg_grid * g, struct bmg_tree * t, opvec * o, int l)
 {
   const span_t all = t->rl[l];
@@ -770,7 +952,7 @@ static void r_relax (bmg_grid * g, struct bmg_tree * t, opvec * o, int l)
   }
   const span_t red = {all.off, t->rl1[l]}, black = {all.off + t->rl1[l], all.n - t->rl1[l]};
   if (red.n) r_push (o, BMG_TI_RELAX, F_DA, 0, 0, t->dlist + red.off, red.n, NULL, 0, 0.);
-  r_boundary (t, o, F_DA, l, 1, SCHED_PRUNED);
+  r_depend (t, o, l);
   if (black.n) r_push (o, BMG_TI_RELAX, F_DA, 0, 0, t->dlist + black.off, black.n, NULL, 0, 0.);
 }
 
@@ -787,10 +969,10 @@ static void r_iteration (bmg_grid * g, struct bmg_tree * t, opvec * o, int nrela
     }
     else if (t->act[l].n)
       r_push (o, BMG_TI_PROLONG, F_DA, 0, 0, t->dlist + t->act[l].off, t->act[l].n, NULL, 0, 0.);
-    r_boundary (t, o, F_DA, l, 1, SCHED_PRUNED);
+    r_depend (t, o, l);
     for (int i = 0; i < nrelax; i++) {
       r_relax (g, t, o, l);
-      r_boundary (t, o, F_DA, l, 1, SCHED_PRUNED);
+      r_depend (t, o, l);
     }
   }
   if (t->leaves.n)
