@@ -142,6 +142,39 @@ int bmg_tree_launch_interp_mixed (const bmg_tree_op * ops, int nops, const bmg_t
                                   const unsigned char * flags, const bmg_tree_coef * coefs,
                                   const bmg_tree_coef32 * coefs32, const bmg_tree_bc * bcs,
                                   unsigned long long * maxres, cudaStream_t st);
+
+/* The cycle of the correction with its cells in distributed shared memory
+   (mg_tree_cycle.cu).  Every cell has a slot: code = rank << 16 | offset,
+   offset 0 of each rank a zero.  Records by level, list and owning rank:
+   own = offset | aux << 16, src = four codes (the prolongation's and a halo
+   cell's coarse cells in bilinear's order, a refined cell's children, a
+   relaxed cell's neighbours x-, x+, y-, y+; a ghost: its interior cell and
+   kind_sides), id = the cell's element index in an all-level field.  aux:
+   the level of a relaxed cell, the kind of a stage's cell. */
+#define BMG_TC_RANKS 16
+#define BMG_TC_STAGES 6
+enum { BMG_TC_PROLONG = 0, BMG_TC_RED, BMG_TC_BLACK, BMG_TC_CELLS };
+enum { BMG_TC_RESTRICT = 0, BMG_TC_HALO, BMG_TC_GHOST };
+typedef struct {
+  uint32_t off[BMG_TC_CELLS + BMG_TC_STAGES][BMG_TC_RANKS], n[BMG_TC_CELLS + BMG_TC_STAGES][BMG_TC_RANKS];
+  int stages, pad_;
+} bmg_tc_level;
+typedef struct {
+  const bmg_tc_level * lv;       /* device, by level */
+  const uint32_t * own, * id;
+  const uint32_t * src;          /* four per record, 16-byte aligned */
+  /* most slots, relaxed cells of a level and stage cells of a level, of a rank */
+  int slots, items, cells, pad_;
+} bmg_tc;
+int bmg_tree_cycle_fits (const bmg_tc * tc, int mixed);
+/* one cycle (red-black, levels minlevel..maxlevel = the tree's depth) and
+   a += da; res restricted */
+int bmg_tree_launch_cycle (const bmg_tc * tc, int minlevel, int maxlevel, int nrelax,
+                           const bmg_tree_levels * T, const double * res, const bmg_tree_coef * coefs,
+                           const bmg_tree_bc * bc, double * a, cudaStream_t st);
+int bmg_tree_launch_cycle_mixed (const bmg_tc * tc, int minlevel, int maxlevel, int nrelax,
+                                 const bmg_tree_levels * T, const float * res, const bmg_tree_coef32 * coefs,
+                                 const bmg_tree_bc * bc, double * a, cudaStream_t st);
 /* dst[k] = (float) src[k], 0 <= k < n */
 int bmg_tree_launch_to_f32 (const double * src, float * dst, long long n, cudaStream_t st);
 

@@ -95,6 +95,10 @@ struct bmg_tree {
   span_t dep[TMAX + 1];
   uint32_t * ddlist;
   bmg_tree_rule * ddrules;
+  /* the cycle in distributed shared memory (mg_tree_cycle.cu); tc.slots = 0:
+     none for this tree */
+  bmg_tc tc;
+  void * dtc[4];                      /* its device arrays: levels, own, id, src */
   bmg_tree_levels T;
   double * dpart;
   int npart;
@@ -142,6 +146,7 @@ static void tree_release (struct bmg_tree * t)
   for (int l = 0; l <= TMAX; l++) { free (t->fl[l]); free (t->nb[l]); }
   cudaFree (t->dflags); cudaFree (t->dlist); cudaFree (t->drules); cudaFree (t->dpart);
   cudaFree (t->dsrules); cudaFree (t->ws32); cudaFree (t->ddlist); cudaFree (t->ddrules);
+  for (int k = 0; k < 4; k++) cudaFree (t->dtc[k]);
   free (t->stages); free (t->deps);
   free (t);
 }
@@ -428,8 +433,161 @@ static int dep_visit (depset * s, int m, int i, int j)
   return d;
 }
 
+/* The records of the cycle in distributed shared memory: a slot of one of
+   the ranks for every cell of the correction, dealt out evenly and in order
+   by level, colour and kind (so that every level's relaxation set, its own
+   cells and the leaves below, is even too), and per level the records of its
+   lists by owning rank.  list, rules: the stages' cells and ghosts.  Leaves
+   tc.slots = 0 when the closure has more stages than a record holds. */
+static int cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h, const uint32_t * list,
+                          const bmg_tree_rule * rules)
+{
+  const int D = t->depth, NR = BMG_TC_RANKS;
+  memset (&t->tc, 0, sizeof t->tc);
+  for (int k = 0; k < 4; k++) { cudaFree (t->dtc[k]); t->dtc[k] = NULL; }
+  long total = 0;
+  for (int l = 0; l <= D; l++) {
+    if (t->dep[l].n > BMG_TC_STAGES) return BMG_OK;
+    total += t->act[l].n + t->rl[l].n;
+    for (long k = 0; k < t->dep[l].n; k++) {
+      const tdep * d = &t->deps[t->dep[l].off + k];
+      total += d->nrest + d->nhalo + d->rules.n;
+    }
+  }
+  int err = 0;
+  uint32_t * slot[TMAX + 1], next[BMG_TC_RANKS];
+  memset (slot, 0, sizeof slot);
+  bmg_tc_level * lv = calloc (D + 1, sizeof *lv);
+  uint32_t * own = malloc ((total + 1)*sizeof (uint32_t)), * id = calloc (total + 1, sizeof (uint32_t));
+  uint32_t * src = malloc ((total + 1)*4*sizeof (uint32_t));
+  if (!lv || !own || !id || !src) err = 1;
+  for (int l = 0; l <= D && !err; l++)
+    if (!(slot[l] = calloc ((size_t) ((1 << l) + 2)*((1 << l) + 2), sizeof (uint32_t)))) err = 1;
+  for (int r = 0; r < NR; r++) next[r] = 1;             /* offset 0: a zero */
+#define LVL(e) ((int) ((e) >> 28))
+#define CI(e) ((int) (((e) >> 14) & 0x3FFF) - 1)
+#define CJ(e) ((int) ((e) & 0x3FFF) - 1)
+#define SLOT(e) slot[LVL (e)][HX (LVL (e), CI (e), CJ (e))]
+  /* active cells: red leaves, black leaves, red refined, black refined */
+  for (int l = 0; l <= D && !err; l++)
+    for (int kind = 0; kind < 4; kind++) {
+      long n = 0, k;
+      for (int pass = 0; pass < 2; pass++) {
+        k = 0;
+        for (long q = 0; q < t->act[l].n; q++) {
+          const uint32_t e = h[t->act[l].off + q];
+          const int leaf = (t->fl[l][HX (l, CI (e), CJ (e))] & BMG_T_LEAF) != 0;
+          if (((CI (e) + CJ (e)) & 1) != (kind & 1) || leaf != !(kind & 2)) continue;
+          if (pass == 1) {
+            const uint32_t r = (uint32_t) (k*NR/n);
+            SLOT (e) = r << 16 | (next[r]++ & 0xffff);
+          }
+          k++;
+        }
+        n = k;
+      }
+    }
+  /* the other cells of the stages, from the finest level's down */
+  for (int l = D; l >= 0 && !err; l--)
+    for (long d = 0; d < t->dep[l].n; d++) {
+      const tdep * q = &t->deps[t->dep[l].off + d];
+      const long m = q->nrest + q->nhalo + q->rules.n;
+      long n = 0, k;
+      for (int pass = 0; pass < 2; pass++) {
+        k = 0;
+        for (long u = 0; u < m; u++) {
+          const uint32_t e = u < q->nrest + q->nhalo ? list[q->off + u]
+            : rules[q->rules.off + u - q->nrest - q->nhalo].ghost;
+          if (SLOT (e)) continue;
+          if (pass == 1) {
+            const uint32_t r = (uint32_t) (k*NR/n);
+            SLOT (e) = r << 16 | (next[r]++ & 0xffff);
+          }
+          k++;
+        }
+        n = k;
+      }
+    }
+  for (int r = 0; r < NR && !err; r++) {
+    if (next[r] > 65535) { err = 2; break; }
+    if ((int) next[r] > t->tc.slots) t->tc.slots = (int) next[r];
+  }
+  /* the code of a source: its slot, or the reader's zero */
+#define CODE(l_, i_, j_, r_) (slot[l_][HX (l_, i_, j_)] ? slot[l_][HX (l_, i_, j_)] : (uint32_t) (r_) << 16)
+  long w = 0;
+  for (int l = 0; l <= D && !err; l++) {
+    lv[l].stages = (int) t->dep[l].n;
+    for (int kind = 0; kind < BMG_TC_CELLS + lv[l].stages; kind++) {
+      const tdep * q = kind >= BMG_TC_CELLS ? &t->deps[t->dep[l].off + kind - BMG_TC_CELLS] : NULL;
+      const uint32_t * cells = kind == BMG_TC_PROLONG ? h + t->act[l].off
+        : kind == BMG_TC_RED ? h + t->rl[l].off : kind == BMG_TC_BLACK ? h + t->rl[l].off + t->rl1[l]
+        : list + q->off;
+      const long n = kind == BMG_TC_PROLONG ? (l > 0 ? t->act[l].n : 0)
+        : kind == BMG_TC_RED ? t->rl1[l] : kind == BMG_TC_BLACK ? t->rl[l].n - t->rl1[l]
+        : q->nrest + q->nhalo + q->rules.n;
+      for (uint32_t r = 0; r < (uint32_t) NR; r++) {
+        lv[l].off[kind][r] = (uint32_t) w;
+        for (long k = 0; k < n; k++) {
+          const int ghost = q && k >= q->nrest + q->nhalo;
+          const bmg_tree_rule * gr = ghost ? &rules[q->rules.off + k - q->nrest - q->nhalo] : NULL;
+          const uint32_t e = ghost ? gr->ghost : cells[k], sl = SLOT (e);
+          if (sl >> 16 != r) continue;
+          const int m = LVL (e), i = CI (e), j = CJ (e);
+          uint32_t * s = src + 4*w;
+          const int halo = q && !ghost && k >= q->nrest;
+          uint32_t aux = 0;
+          if (ghost) {
+            s[0] = SLOT (gr->inner); s[1] = gr->kind_sides; s[2] = s[3] = 0;
+            aux = BMG_TC_GHOST;
+          }
+          else if (kind == BMG_TC_PROLONG || halo) {
+            const int pi = i >> 1, pj = j >> 1, cx = (i & 1) ? 1 : -1, cy = (j & 1) ? 1 : -1;
+            s[0] = CODE (m - 1, pi, pj, r); s[1] = CODE (m - 1, pi + cx, pj, r);
+            s[2] = CODE (m - 1, pi, pj + cy, r); s[3] = CODE (m - 1, pi + cx, pj + cy, r);
+            aux = BMG_TC_HALO;
+          }
+          else if (q) {
+            for (int c = 0; c < 4; c++) s[c] = CODE (m + 1, 2*i + (c >> 1), 2*j + (c & 1), r);
+            aux = BMG_TC_RESTRICT;
+          }
+          else {
+            s[0] = CODE (m, i - 1, j, r); s[1] = CODE (m, i + 1, j, r);
+            s[2] = CODE (m, i, j - 1, r); s[3] = CODE (m, i, j + 1, r);
+            id[w] = (uint32_t) (g->off64[m] + (size_t) (i + 1)*g->g64[m].P + g->g64[m].xo + j);
+            aux = (uint32_t) m;
+          }
+          own[w++] = (sl & 0xffff) | aux << 16;
+        }
+        lv[l].n[kind][r] = (uint32_t) (w - lv[l].off[kind][r]);
+      }
+    }
+    for (int r = 0; r < NR; r++) {
+      const int n = (int) (lv[l].n[BMG_TC_RED][r] + lv[l].n[BMG_TC_BLACK][r]);
+      if (n > t->tc.items) t->tc.items = n;
+      int c = 0;
+      for (int st = 0; st < lv[l].stages; st++) c += (int) lv[l].n[BMG_TC_CELLS + st][r];
+      if (c > t->tc.cells) t->tc.cells = c;
+    }
+  }
+#undef CODE
+#undef SLOT
+#undef LVL
+#undef CI
+#undef CJ
+  const size_t sz[4] = {(D + 1)*sizeof *lv, total*sizeof (uint32_t), total*sizeof (uint32_t), total*4*sizeof (uint32_t)};
+  const void * hp[4] = {lv, own, id, src};
+  for (int k = 0; k < 4 && !err; k++)
+    if (cudaMalloc (&t->dtc[k], sz[k] + 16) != cudaSuccess ||
+        cudaMemcpy (t->dtc[k], hp[k], sz[k], cudaMemcpyHostToDevice) != cudaSuccess) err = 1;
+  t->tc.lv = t->dtc[0]; t->tc.own = t->dtc[1]; t->tc.id = t->dtc[2]; t->tc.src = t->dtc[3];
+  if (err) { cudaGetLastError (); t->tc.slots = 0; }
+  for (int l = 0; l <= D; l++) free (slot[l]);
+  free (lv); free (own); free (id); free (src);
+  return err == 1 ? BMG_ENOMEM : BMG_OK;
+}
+
 /* the stages of every level, uploaded; h: the host cell lists */
-static int depend (struct bmg_tree * t, const uint32_t * h)
+static int depend (bmg_grid * g, struct bmg_tree * t, const uint32_t * h)
 {
   depset s;
   memset (&s, 0, sizeof s);
@@ -513,8 +671,9 @@ static int depend (struct bmg_tree * t, const uint32_t * h)
        (nrules && cudaMemcpy (t->ddrules, rules, nrules*sizeof (bmg_tree_rule), cudaMemcpyHostToDevice)
         != cudaSuccess)))
     s.err = 1;
+  int r = s.err ? BMG_ENOMEM : cycle_records (g, t, h, list, rules);
   free (list); free (rules);
-  return s.err ? BMG_ENOMEM : BMG_OK;
+  return r;
 }
 
 /* flags of halo cells and prolongation leaves, cell lists, ghost rules:
@@ -634,7 +793,7 @@ static int derive (bmg_grid * g, struct bmg_tree * t)
       cudaMemcpy (t->dlist, h, total*sizeof (uint32_t), cudaMemcpyHostToDevice) != cudaSuccess ||
       (k && cudaMemcpy (t->drules, hr, k*sizeof (bmg_tree_rule), cudaMemcpyHostToDevice) != cudaSuccess))
     st = BMG_ENOMEM;
-  if (!st) st = depend (t, h);
+  if (!st) st = depend (g, t, h);
   free (h); free (hf);
   if (st) { free (hr); return FAIL (st); }
   /* boundary schedules */
@@ -956,12 +1115,15 @@ static void r_relax (bmg_grid * g, struct bmg_tree * t, opvec * o, int l)
   if (black.n) r_push (o, BMG_TI_RELAX, F_DA, 0, 0, t->dlist + black.off, black.n, NULL, 0, 0.);
 }
 
+/* the operations of an iteration; *cyc0 .. *cyc1: those of the correction's
+   cycle, a += da included */
 static void r_iteration (bmg_grid * g, struct bmg_tree * t, opvec * o, int nrelax, int minlevel,
-                         int maxlevel)
+                         int maxlevel, long * cyc0, long * cyc1)
 {
   for (int m = t->depth - 1; m >= 0; m--)
     if (t->ref[m].n)
       r_push (o, BMG_TI_RESTRICT, F_RES, 0, 0, t->dlist + t->ref[m].off, t->ref[m].n, NULL, 0, 0.);
+  *cyc0 = o->n;
   for (int l = minlevel; l <= maxlevel; l++) {
     if (l == minlevel) {
       if (t->rl[l].n)
@@ -977,6 +1139,7 @@ static void r_iteration (bmg_grid * g, struct bmg_tree * t, opvec * o, int nrela
   }
   if (t->leaves.n)
     r_push (o, BMG_TI_ADD, F_A, 0, 0, t->dlist + t->leaves.off, t->leaves.n, NULL, 0, 0.);
+  *cyc1 = o->n;
   r_boundary (t, o, F_A, t->depth, 0, SCHED_FULL);
   if (t->leaves.n)
     r_push (o, BMG_TI_RESIDUAL, F_RES, 0, 0, t->dlist + t->leaves.off, t->leaves.n, NULL, 0, 0.);
@@ -988,6 +1151,16 @@ static int read_max (bmg_grid * g, double * m)
   CKT (cudaStreamSynchronize (g->stream));
   *m = g->h_pinned[0];
   return BMG_OK;
+}
+
+/* whether the cycle runs in distributed shared memory: red-black, to the
+   tree's depth, and the correction's cells fit.  The depth-10 band tree
+   takes 140 ms per solve this way and 284 ms as interpreted
+   operations. */
+static int cycle_fits (const bmg_grid * g, const struct bmg_tree * t, const tkey * key)
+{
+  return g->relax == BMG_RELAX_RBGS && t->tc.slots > 0 && key->nrelax > 0 &&
+    key->minlevel <= key->maxlevel && key->maxlevel == t->depth && bmg_tree_cycle_fits (&t->tc, key->mixed);
 }
 
 /* one mg_solve iteration (cycle, residual, maximum to pinned memory),
@@ -1015,7 +1188,8 @@ static int t_iteration (bmg_grid * g, struct bmg_tree * t, const tkey * key, dou
     /* the iteration as one interpreter launch, its operations uploaded once */
     graph_drop (victim);
     opvec o = {NULL, 0, 0, 0, 0., c->ax.p != NULL, c->lam.p != NULL, 8.};
-    r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel);
+    long cyc0, cyc1;
+    r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel, &cyc0, &cyc1);
     victim->bytes = o.bytes;
     if (o.err) { free (o.v); return FAIL (BMG_ENOMEM); }
     if (cudaMalloc ((void **) &victim->dops, (o.n + 1)*sizeof (bmg_tree_op)) != cudaSuccess ||
@@ -1034,9 +1208,18 @@ static int t_iteration (bmg_grid * g, struct bmg_tree * t, const tkey * key, dou
     cudaGraph_t graph;
     CKT (cudaStreamBeginCapture (g->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t me = cudaMemsetAsync (g->d_maxres, 0, sizeof (unsigned long long), g->stream);
-    int r = me == cudaSuccess ?
-      bmg_tree_launch_interp (victim->dops, (int) victim->nops, &t->T, fields, b, t->dflags, co,
-                              bcs, g->d_maxres, g->stream) : (int) me;
+    int r = (int) me;
+    const int fast = cycle_fits (g, t, key);
+    const long n = victim->nops;
+    if (!r)
+      r = bmg_tree_launch_interp (victim->dops, (int) (fast ? cyc0 : n), &t->T, fields, b, t->dflags, co,
+                                  bcs, g->d_maxres, g->stream);
+    if (!r && fast)
+      r = bmg_tree_launch_cycle (&t->tc, key->minlevel, key->maxlevel, key->nrelax, &t->T, res, co, abc,
+                                 a, g->stream);
+    if (!r && fast)
+      r = bmg_tree_launch_interp (victim->dops + cyc1, (int) (n - cyc1), &t->T, fields, b, t->dflags, co,
+                                  bcs, g->d_maxres, g->stream);
     me = cudaMemcpyAsync (g->h_pinned, g->d_maxres, sizeof (double), cudaMemcpyDeviceToHost,
                           g->stream);
     cudaError_t ee = cudaStreamEndCapture (g->stream, &graph);
@@ -1052,7 +1235,7 @@ static int t_iteration (bmg_grid * g, struct bmg_tree * t, const tkey * key, dou
     cudaGraphDestroy (graph);
     CKT (ie);
     victim->key = *key;
-    victim->launches = 1;
+    victim->launches = fast ? 3 : 1;
     victim->valid = 1;
     e = victim;
   }
@@ -1061,7 +1244,8 @@ static int t_iteration (bmg_grid * g, struct bmg_tree * t, const tkey * key, dou
     {
       /* the same iteration's algorithmic bytes, from its operation list */
       opvec o = {NULL, 0, 0, 0, 0., c->ax.p != NULL, c->lam.p != NULL, 8.};
-      r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel);
+      long cyc0, cyc1;
+    r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel, &cyc0, &cyc1);
       victim->bytes = o.bytes;
       free (o.v);
     }
@@ -1106,7 +1290,8 @@ static int t_iteration_mixed (bmg_grid * g, struct bmg_tree * t, const tkey * ke
   if (!e) {
     graph_drop (victim);
     opvec o = {NULL, 0, 0, 0, 0., c->ax.p != NULL, c->lam.p != NULL, 4.};
-    r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel);
+    long cyc0, cyc1;
+    r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel, &cyc0, &cyc1);
     victim->bytes = o.bytes;
     if (o.err) { free (o.v); return FAIL (BMG_ENOMEM); }
     if (cudaMalloc ((void **) &victim->dops, (o.n + 1)*sizeof (bmg_tree_op)) != cudaSuccess ||
@@ -1124,9 +1309,18 @@ static int t_iteration_mixed (bmg_grid * g, struct bmg_tree * t, const tkey * ke
     cudaGraph_t graph;
     CKT (cudaStreamBeginCapture (g->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t me = cudaMemsetAsync (g->d_maxres, 0, sizeof (unsigned long long), g->stream);
-    int r = me == cudaSuccess ?
-      bmg_tree_launch_interp_mixed (victim->dops, (int) victim->nops, &t->T, a, f32, b,
-                                    t->dflags, co, c32, bcs, g->d_maxres, g->stream) : (int) me;
+    int r = (int) me;
+    const int fast = cycle_fits (g, t, key);
+    const long n = victim->nops;
+    if (!r)
+      r = bmg_tree_launch_interp_mixed (victim->dops, (int) (fast ? cyc0 : n), &t->T, a, f32, b,
+                                        t->dflags, co, c32, bcs, g->d_maxres, g->stream);
+    if (!r && fast)
+      r = bmg_tree_launch_cycle_mixed (&t->tc, key->minlevel, key->maxlevel, key->nrelax, &t->T, f32[1],
+                                       c32, abc, a, g->stream);
+    if (!r && fast)
+      r = bmg_tree_launch_interp_mixed (victim->dops + cyc1, (int) (n - cyc1), &t->T, a, f32, b,
+                                        t->dflags, co, c32, bcs, g->d_maxres, g->stream);
     me = cudaMemcpyAsync (g->h_pinned, g->d_maxres, sizeof (double), cudaMemcpyDeviceToHost,
                           g->stream);
     cudaError_t ee = cudaStreamEndCapture (g->stream, &graph);
@@ -1142,7 +1336,7 @@ static int t_iteration_mixed (bmg_grid * g, struct bmg_tree * t, const tkey * ke
     cudaGraphDestroy (graph);
     CKT (ie);
     victim->key = *key;
-    victim->launches = 1;
+    victim->launches = fast ? 3 : 1;
     victim->valid = 1;
     e = victim;
   }
