@@ -273,6 +273,40 @@ __device__ __forceinline__ T relax_value (const bmg_geom & g, long long id, cons
   return nn/d;
 }
 
+/* ---------------------------------------------------------------- */
+/* quotients by a divisor known in advance                           */
+/* ---------------------------------------------------------------- */
+
+/* n/d in IEEE double precision (round to nearest) from y = 1/d, itself
+   correctly rounded: the first quotient n*y is within 2^-52 of n/d, one
+   correction makes it faithful (the error left before its rounding is below
+   2^-104), and a second correction of a faithful quotient, whose residual is
+   exact, rounds to nearest (P. Markstein, Computation of elementary functions
+   on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).  Five
+   dependent operations without a branch, about 50 cycles that overlap with
+   those of the thread's other cells; the division instruction sequence takes
+   112 and does not.  Exact for positive d and |n| in [2^-450, 2^450], and
+   for n = +-0 (the signs of the corrections keep that of zero); for other
+   operands quotient_unsafe () / divisor_unsafe () tell that a plain
+   division is needed (by a warp vote, off the quotient's critical path). */
+__device__ __forceinline__ double exact_quotient (double n, double d, double y)
+{
+  const double q0 = n*y;
+  const double q1 = fma (-fma (d, q0, -n), y, q0);
+  return fma (-fma (d, q1, -n), y, q1);
+}
+
+__device__ __forceinline__ bool quotient_unsafe (double n)
+{
+  const unsigned h = (unsigned) __double2hiint (n) & 0x7fffffffu;
+  return h - 0x23d00000u > 0x38400000u && (h | (unsigned) __double2loint (n)) != 0u;
+}
+
+__device__ __forceinline__ bool divisor_unsafe (double d)
+{
+  return (unsigned) __double2hiint (d) - 0x23d00000u > 0x38400000u;
+}
+
 /* x/Delta; when Delta is a power of two (L0 = 1, Delta = 2^-l) the
    division is an exact scaling and x*(1/Delta) is the same double, at a
    fraction of the cost of the IEEE division */

@@ -40,6 +40,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
 #include "mg_device.cuh"
 
 using namespace bmgd;
@@ -1400,7 +1401,8 @@ k_relax_tile2d_x4 (bmg_geom g, double * __restrict__ out, const double * __restr
    the same strips, exchanges and barriers, eight cells per thread (four
    of each colour) whose exact coefficients and -Delta^2 b stay in
    registers, and every update in relax_value's expression and order with
-   the IEEE division (as k_relax_tile2d_x4), so that the result is
+   the quotient of exact_quotient () (four of them overlap in a thread, four
+   divisions do not), so that the result is
    bit-identical to the single-CTA bottom and the tile launches it
    replaces; the fused prolongation is bilinear's expression in FP64. */
 namespace clx {
@@ -1435,8 +1437,10 @@ k_level_cluster_x (bmg_geom g, double * __restrict__ out, const double * __restr
   const double D2 = Delta*Delta;
   pdl_trigger ();
 
-  /* the exact coefficients of the thread's eight cells */
-  double cxl[2][4], cxu[2][4], cyl[2][4], cyr[2][4], cnb[2][4], cdl[2][LAM ? 4 : 1];
+  /* the exact coefficients of the thread's eight cells, their diagonals
+     and the diagonals' reciprocals (exact_quotient) */
+  double cxl[2][4], cxu[2][4], cyl[2][4], cyr[2][4], cnb[2][4], cd[2][4], cy[2][4];
+  bool bad = false;
   {
     double r8[8], xl8[8], xu8[8], yl8[9], l8[8];
 #pragma unroll
@@ -1483,10 +1487,14 @@ k_level_cluster_x (bmg_geom g, double * __restrict__ out, const double * __restr
         cxl[c][e] = odd ? xl8[2*e + 1] : xl8[2*e]; cxu[c][e] = odd ? xu8[2*e + 1] : xu8[2*e];
         cyl[c][e] = odd ? yl8[2*e + 1] : yl8[2*e]; cyr[c][e] = odd ? yl8[2*e + 2] : yl8[2*e + 1];
         cnb[c][e] = (-D2)*(odd ? r8[2*e + 1] : r8[2*e]);
-        if (LAM) cdl[c][LAM ? e : 0] = (-(odd ? l8[2*e + 1] : l8[2*e]))*D2;
+        double d = (-(LAM ? (odd ? l8[2*e + 1] : l8[2*e]) : lam.c))*D2;
+        d += cxu[c][e] + cxl[c][e];
+        d += cyr[c][e] + cyl[c][e];
+        cd[c][e] = d;
+        cy[c][e] = rowok ? 1./d : 0.;
+        bad = bad || (rowok && divisor_unsafe (d));
       }
   }
-  const double dlc = (-lam.c)*D2;
 
   const bool rowghost_lo = !px && gi == 0 && p >= 1, rowghost_hi = !px && gi == N - 1 && p <= BYR - 2;
   const double frow = rowghost_lo ? (double) bc.fac[1] : (double) bc.fac[0];
@@ -1600,13 +1608,21 @@ k_level_cluster_x (bmg_geom g, double * __restrict__ out, const double * __restr
 #pragma unroll
           for (int e = 0; e < 4; e++) {
             /* relax_value's expression and order (poisson.h:303-319) */
-            double d = LAM ? cdl[c][LAM ? e : 0] : dlc;
-            d += cxu[c][e] + cxl[c][e];
-            d += cyr[c][e] + cyl[c][e];
             double nn = cnb[c][e] + (cxu[c][e]*dnv[e] + cxl[c][e]*upv[e]);
-            nn = nn + (cyr[c][e]*v[e + 1] + cyl[c][e]*v[e]);
-            nv[e] = nn/d;
+            nv[e] = nn + (cyr[c][e]*v[e + 1] + cyl[c][e]*v[e]);
           }
+          bool plain = bad;
+          double q[4];
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            plain = plain || quotient_unsafe (nv[e]);
+            q[e] = exact_quotient (nv[e], cd[c][e], cy[c][e]);
+          }
+          if (__any_sync (__activemask (), plain))
+#pragma unroll
+            for (int e = 0; e < 4; e++) q[e] = nv[e]/cd[c][e];
+#pragma unroll
+          for (int e = 0; e < 4; e++) nv[e] = q[e];
           const unsigned aw = sbase + 8u*(c*SAW + p*MP + OFS + m0);
           sts_d2 (aw, make_double2 (nv[0], nv[1]));
           sts_d2 (aw + 16, make_double2 (nv[2], nv[3]));
@@ -1845,11 +1861,31 @@ __device__ __forceinline__ void bot_restrict (const bmg_geom & gf, const void * 
   }
 }
 
+/* the bilinear prolongation of fine cell (i, j, k) (multigrid-common.h:124-140) */
+template <int DIM, typename TC>
+__device__ __forceinline__ TC bot_bilinear (const bmg_geom & gc, const TC * s, int i, int j, int k)
+{
+  const int pi = i >> 1, cx = (i & 1) ? 1 : -1;
+  if (DIM == 1)
+    return (TC(3)*s[cidx<1> (gc, pi, 0, 0)] + s[cidx<1> (gc, pi + cx, 0, 0)])/TC(4);
+  const int pj = j >> 1, cy = (j & 1) ? 1 : -1;
+  if (DIM == 2)
+    return (TC(9)*s[cidx<2> (gc, pi, pj, 0)] +
+            TC(3)*(s[cidx<2> (gc, pi + cx, pj, 0)] + s[cidx<2> (gc, pi, pj + cy, 0)]) +
+            s[cidx<2> (gc, pi + cx, pj + cy, 0)])/TC(16);
+  const int pk = k >> 1, cz = (k & 1) ? 1 : -1;
+  return (TC(27)*s[cidx<3> (gc, pi, pj, pk)] +
+          TC(9)*(s[cidx<3> (gc, pi + cx, pj, pk)] + s[cidx<3> (gc, pi, pj + cy, pk)] +
+                 s[cidx<3> (gc, pi, pj, pk + cz)]) +
+          TC(3)*(s[cidx<3> (gc, pi + cx, pj + cy, pk)] + s[cidx<3> (gc, pi + cx, pj, pk + cz)] +
+                 s[cidx<3> (gc, pi, pj + cy, pk + cz)]) +
+          s[cidx<3> (gc, pi + cx, pj + cy, pk + cz)])/TC(64);
+}
+
 template <int DIM, typename TC, typename TF>
 __device__ __forceinline__ void bot_prolong (const bmg_geom & gc, const void * cv, const bmg_geom & gf, void * fv,
                              const BCH & bc, int zero)
 {
-  const TC * s = (const TC *) cv;
   TF * f = (TF *) fv;
   const int n = gf.n;
   const long long total = DIM == 1 ? n : DIM == 2 ? (long long) n*n : (long long) n*n*n;
@@ -1859,29 +1895,7 @@ __device__ __forceinline__ void bot_prolong (const bmg_geom & gc, const void * c
     if (DIM == 1) i = qq;
     else if (DIM == 2) { i = qq >> ln; j = qq & (n - 1); }
     else { i = qq >> (2*ln); j = (qq >> ln) & (n - 1); k = qq & (n - 1); }
-    TC v = TC(0);
-    if (!zero) {
-      const int pi = i >> 1, cx = (i & 1) ? 1 : -1;
-      if (DIM == 1)
-        v = (TC(3)*s[cidx<1> (gc, pi, 0, 0)] + s[cidx<1> (gc, pi + cx, 0, 0)])/TC(4);
-      else if (DIM == 2) {
-        const int pj = j >> 1, cy = (j & 1) ? 1 : -1;
-        v = (TC(9)*s[cidx<2> (gc, pi, pj, 0)] +
-             TC(3)*(s[cidx<2> (gc, pi + cx, pj, 0)] + s[cidx<2> (gc, pi, pj + cy, 0)]) +
-             s[cidx<2> (gc, pi + cx, pj + cy, 0)])/TC(16);
-      }
-      else {
-        const int pj = j >> 1, cy = (j & 1) ? 1 : -1;
-        const int pk = k >> 1, cz = (k & 1) ? 1 : -1;
-        v = (TC(27)*s[cidx<3> (gc, pi, pj, pk)] +
-             TC(9)*(s[cidx<3> (gc, pi + cx, pj, pk)] + s[cidx<3> (gc, pi, pj + cy, pk)] +
-                    s[cidx<3> (gc, pi, pj, pk + cz)]) +
-             TC(3)*(s[cidx<3> (gc, pi + cx, pj + cy, pk)] + s[cidx<3> (gc, pi + cx, pj, pk + cz)] +
-                    s[cidx<3> (gc, pi, pj + cy, pk + cz)]) +
-             s[cidx<3> (gc, pi + cx, pj + cy, pk + cz)])/TC(64);
-      }
-    }
-    const TF w = (TF) v;
+    const TF w = zero ? TF(0) : (TF) bot_bilinear<DIM, TC> (gc, (const TC *) cv, i, j, k);
     f[cidx<DIM> (gf, i, j, k)] = w;
     ghosts_homog<DIM, TF> (f, gf, i, j, k, w, bc);
   }
@@ -2030,19 +2044,123 @@ __device__ __forceinline__ void bot_sweeps2d (const bmg_geom g, T * a, const T *
     }
 }
 
-/* all nrelax sweeps of one 2D level of the mixed form whose cells of one
-   colour number at most K nt: each thread keeps its (up to K per colour)
-   cells' coefficients in registers, divided by the diagonal once per
-   level, so a pass reads only the four neighbours of each cell from shared
-   memory and needs no division: a = beta + sum of w a_neighbour with
-   w = alpha/d and beta = -Delta^2 b/d, the relaxation of relax_value
-   (poisson.h:303-319) up to rounding.  The pass is bound by the
-   shared-memory bandwidth of the one SM, which this cuts from nine operands
-   per cell to four. */
 __device__ __forceinline__ float fma_t (float a, float b, float c) { return fmaf (a, b, c); }
 __device__ __forceinline__ double fma_t (double a, double b, double c) { return fma (a, b, c); }
 
-template <typename T, int K, bool EXACT>
+/* The initial iterate and all nrelax sweeps of one staged level whose cells
+   of a colour number at most the block's threads (up to 32^2, 8^3), in any
+   form: each thread owns one cell of each colour, with its coefficients in
+   registers, takes their initial values (init: zero, or the prolongation of
+   the level below), and the level is held split by colour without ghost
+   cells, so that a warp's accesses are consecutive.  A box ghost is +-1 times
+   the cell it mirrors, which only that cell reads: its term is the cell's own
+   value with the weight's sign (exact), and no pass writes ghosts; they are
+   written once at the end, with the padded array.  Only the threads that own
+   cells meet at the pass's barrier.
+     EXACT: relax_value's expression and order, in double precision with the
+   quotient by the cell's diagonal from its reciprocal (exact_quotient).
+   Otherwise (mixed form, two dimensions) the weights are divided by the
+   diagonal once per level: a = beta + sum of w a_neighbour.
+   Bound: the latency of a pass (loads, the sum, the quotient, a barrier).
+   With the quotients in the cluster kernels too: 512^2 FP64 solve 26.3 ->
+   25.6 ms, 64^3 mixed solve 1.27 -> 1.23 ms, 128^2 FP64 solve 641 -> 619 us. */
+template <int DIM, typename T, bool EXACT, typename I>
+__device__ __forceinline__ void bot_sweeps_own (const bmg_geom g, T * a, const T * b, const T * ax,
+                                                const T * ay, const T * az, T axc, T ayc, T azc,
+                                                const T * lam, T lamc, T D2, const BCH bc, int nrelax,
+                                                I init)
+{
+  const int n = g.n, ln = 31 - __clz (n), nh = n >> 1, half = (1 << (DIM*ln)) >> 1;
+  const int tid = threadIdx.x, active = half < 32 ? 32 : half;
+  const bool own = tid < half;
+  T w[2][2*DIM], be[2], d[2], y[2], v[2];
+  int nb[2][2*DIM];                                   /* slots: upper, lower per direction */
+  int ci[2], cj[2], ck[2];
+  bool plain = false;                                 /* a diagonal outside exact_quotient's range */
+  if (own)
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    const int row = tid >> (ln - 1), h = tid & (nh - 1);
+    int x[3] = {DIM == 2 ? row : row >> ln, DIM == 2 ? 0 : row & (n - 1), 0};
+    x[DIM - 1] = 2*h + ((c + x[0] + (DIM == 3 ? x[1] : 0)) & 1);
+    ci[c] = x[0]; cj[c] = x[1]; ck[c] = x[2];
+    v[c] = init (x[0], x[1], x[2]);
+    const int id = (int) cidx<DIM> (g, x[0], x[1], x[2]);
+    T dd = (-(lam ? lam[id] : lamc))*D2;
+    be[c] = (-D2)*b[id];
+#pragma unroll
+    for (int e = 0; e < DIM; e++) {
+      const T * al = e == 0 ? ax : e == 1 ? ay : az;
+      const T alc = e == 0 ? axc : e == 1 ? ayc : azc;
+      const T w1 = al ? al[id + (int) cstride<DIM> (g, e)] : alc, w0 = al ? al[id] : alc;
+      dd += w1 + w0;
+#pragma unroll
+      for (int lo = 0; lo < 2; lo++) {
+        const bool edge = x[e] == (lo ? 0 : n - 1), box = edge && !bc.periodic[e];
+        const T wv = lo ? w0 : w1;
+        w[c][2*e + lo] = box && bc.fac[2*e + lo] < 0 ? -wv : wv;
+        int z[3] = {x[0], x[1], x[2]};
+        z[e] = edge ? (lo ? n - 1 : 0) : x[e] + (lo ? -1 : 1);
+        const int r = DIM == 2 ? z[0] : (z[0] << ln) + z[1];
+        nb[c][2*e + lo] = box ? c*half + tid : (c ^ 1)*half + r*nh + (z[DIM - 1] >> 1);
+      }
+    }
+    d[c] = dd;
+    if (EXACT && sizeof (T) == 4) continue;           /* plain divisions */
+    y[c] = T(1)/dd;
+    if (EXACT) plain = plain || divisor_unsafe ((double) dd);
+    else {
+#pragma unroll
+      for (int e = 0; e < 2*DIM; e++) w[c][e] = w[c][e]*y[c];
+      be[c] = be[c]*y[c];
+    }
+  }
+  /* the level split by colour, in the place of its padded array */
+  if (own) { a[tid] = v[0]; a[half + tid] = v[1]; }
+  __syncthreads ();
+  if (tid < active)
+    for (int sw = 0; sw < nrelax; sw++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        if (own) {
+          T m = be[c];
+          if (EXACT) {
+#pragma unroll
+            for (int e = 0; e < DIM; e++)
+              m = m + (w[c][2*e]*a[nb[c][2*e]] + w[c][2*e + 1]*a[nb[c][2*e + 1]]);
+            if (sizeof (T) == 4) v[c] = m/d[c];
+            else {
+              v[c] = (T) exact_quotient ((double) m, (double) d[c], (double) y[c]);
+              if (__any_sync (__activemask (), plain || quotient_unsafe ((double) m))) v[c] = m/d[c];
+            }
+          }
+          else {
+#pragma unroll
+            for (int e = 0; e < 2*DIM; e++) m = fma_t (w[c][e], a[nb[c][e]], m);
+            v[c] = m;
+          }
+          a[c*half + tid] = v[c];
+        }
+        if (active <= 32) __syncwarp ();
+        else asm volatile ("bar.sync 1, %0;" :: "r"(active) : "memory");
+      }
+  __syncthreads ();
+  if (own)
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      a[cidx<DIM> (g, ci[c], cj[c], ck[c])] = v[c];
+      if (DIM == 2) ghosts_homog_2d<T> (a, g, ci[c], cj[c], v[c], bc);
+      else ghosts_homog<DIM, T> (a, g, ci[c], cj[c], ck[c], v[c], bc);
+    }
+}
+
+/* all nrelax sweeps of one 2D level of the mixed form with more cells of a
+   colour than threads, at most K nt: each thread keeps its (up to K per
+   colour) cells' coefficients in registers, divided by the diagonal once
+   per level, so a pass reads only the four neighbours of each cell from
+   shared memory and needs no division (the relaxation of relax_value,
+   poisson.h:303-319, up to rounding). */
+template <typename T, int K>
 __device__ __forceinline__ void bot_sweeps2d_reg (const bmg_geom g, T * a, const T * b,
                                                   const T * ax, const T * ay, T axc,
                                                   T ayc, const T * lam, T lamc,
@@ -2082,22 +2200,14 @@ __device__ __forceinline__ void bot_sweeps2d_reg (const bmg_geom g, T * a, const
         const int e = (i + 1)*P + 1 + j;
         const T x0 = ax ? ax[e] : axc, x1 = ax ? ax[e + P] : axc;
         const T y0 = ay ? ay[e] : ayc, y1 = ay ? ay[e + 1] : ayc;
-        if (EXACT) {
-          /* the plain form: the coefficients as they are, and -Delta^2 b */
-          wx0[c][k] = x0; wx1[c][k] = x1; wy0[c][k] = y0; wy1[c][k] = y1;
-          beta[c][k] = (-D2)*b[e];
-        }
-        else {
-          T d = (-(lam ? lam[e] : lamc))*D2;
-          d += x1 + x0;
-          d += y1 + y0;
-          const T inv = T(1)/d;
-          wx0[c][k] = x0*inv; wx1[c][k] = x1*inv; wy0[c][k] = y0*inv; wy1[c][k] = y1*inv;
-          beta[c][k] = ((-D2)*b[e])*inv;
-        }
+        T d = (-(lam ? lam[e] : lamc))*D2;
+        d += x1 + x0;
+        d += y1 + y0;
+        const T inv = T(1)/d;
+        wx0[c][k] = x0*inv; wx1[c][k] = x1*inv; wy0[c][k] = y0*inv; wy1[c][k] = y1*inv;
+        beta[c][k] = ((-D2)*b[e])*inv;
       }
     }
-  const T dl = (-lamc)*D2;                    /* lambda constant in the exact form */
   for (int sw = 0; sw < nrelax; sw++)
 #pragma unroll
     for (int c = 0; c < 2; c++) {
@@ -2107,18 +2217,8 @@ __device__ __forceinline__ void bot_sweeps2d_reg (const bmg_geom g, T * a, const
       for (int k = 0; k < K; k++) {
         const int t = ij[c][k] < 0 ? 0 : ij[c][k];
         e[k] = ((t >> 16) + 1)*P + 1 + (t & 0xffff);
-        if (EXACT) {
-          /* relax_value's expression and order (poisson.h:303-319) */
-          T d = dl;
-          d += wx1[c][k] + wx0[c][k];
-          d += wy1[c][k] + wy0[c][k];
-          T m = beta[c][k] + (wx1[c][k]*a[e[k] + P] + wx0[c][k]*a[e[k] - P]);
-          m = m + (wy1[c][k]*a[e[k] + 1] + wy0[c][k]*a[e[k] - 1]);
-          v[k] = m/d;
-        }
-        else
-          v[k] = fma_t (wy0[c][k], a[e[k] - 1], fma_t (wy1[c][k], a[e[k] + 1],
-                 fma_t (wx0[c][k], a[e[k] - P], fma_t (wx1[c][k], a[e[k] + P], beta[c][k]))));
+        v[k] = fma_t (wy0[c][k], a[e[k] - 1], fma_t (wy1[c][k], a[e[k] + 1],
+               fma_t (wx0[c][k], a[e[k] - P], fma_t (wx1[c][k], a[e[k] + P], beta[c][k]))));
       }
 #pragma unroll
       for (int k = 0; k < K; k++)
@@ -2150,22 +2250,10 @@ __device__ __forceinline__ void bot_level2d (const bmg_geom g, void * dav, const
     * lam = (const T *) lamv;
   const T D2 = (T) Delta*(T) Delta;
   /* up to four cells per colour per thread in FP32, two in FP64
-     (registers); one where the level's cells of a colour fit the threads,
-     so that the small levels' passes carry no empty slots */
+     (registers) */
   constexpr int K = sizeof (T) == 4 ? 4 : 2;
-  if (fast && g.n >= 2 && g.n*(g.n >> 1) <= nt) {
-    bot_sweeps2d_reg<T, 1, false> (g, a, b, ax, ay, (T) axc, (T) ayc, lam, (T) lamc, D2, bc, nrelax, nt, small);
-    return;
-  }
   if (fast && g.n >= 2 && g.n*(g.n >> 1) <= K*nt) {
-    bot_sweeps2d_reg<T, K, false> (g, a, b, ax, ay, (T) axc, (T) ayc, lam, (T) lamc, D2, bc, nrelax, nt, small);
-    return;
-  }
-  /* the plain FP64 form with lambda constant, on the levels whose cells of
-     a colour fit the threads: the same register ownership with the exact
-     coefficients, in the reference's evaluation order */
-  if (!fast && sizeof (T) == 8 && !lam && g.n >= 2 && g.n*(g.n >> 1) <= nt) {
-    bot_sweeps2d_reg<T, 1, true> (g, a, b, ax, ay, (T) axc, (T) ayc, lam, (T) lamc, D2, bc, nrelax, nt, small);
+    bot_sweeps2d_reg<T, K> (g, a, b, ax, ay, (T) axc, (T) ayc, lam, (T) lamc, D2, bc, nrelax, nt, small);
     return;
   }
   if (ax && lam)
@@ -2196,6 +2284,38 @@ __device__ __forceinline__ void bot_prolong_st (int stc, const bmg_geom & gc, co
   else if (stc == BMG_ST_F32 && stf == BMG_ST_F32) bot_prolong<DIM, float, float> (gc, c, gf, f, bc, zero);
   else if (stc == BMG_ST_F64 && stf == BMG_ST_F32) bot_prolong<DIM, double, float> (gc, c, gf, f, bc, zero);
   else bot_prolong<DIM, float, double> (gc, c, gf, f, bc, zero);
+}
+
+/* level m of the bottom by bot_sweeps_own (out of line: its registers are
+   not those of the larger levels' sweeps) */
+template <int DIM, typename T>
+__device__ __noinline__ void bot_own_level (const BotParams & P, int m, unsigned char * bsm)
+{
+  const BotLevel & L = P.lv[m];
+  const BotStage & S = P.sm[m];
+  const bool zero = m == 0;
+  const BotStage & Sc = P.sm[zero ? 0 : m - 1];
+  const bmg_geom gc = Sc.gs;
+  const void * cda = sm_at (bsm, Sc.off_da);
+  const int stc = P.lv[zero ? 0 : m - 1].st;
+  auto init = [=] (int i, int j, int k) -> T {
+    if (zero) return T(0);
+    return stc == BMG_ST_F64 ? (T) bot_bilinear<DIM, double> (gc, (const double *) cda, i, j, k)
+      : (T) bot_bilinear<DIM, float> (gc, (const float *) cda, i, j, k);
+  };
+  const T * ax = (const T *) sm_at (bsm, S.off_alpha[0]), * ay = (const T *) sm_at (bsm, S.off_alpha[1]);
+  const T * az = DIM == 3 ? (const T *) sm_at (bsm, S.off_alpha[2]) : NULL;
+  const T * lam = (const T *) sm_at (bsm, S.off_lambda), * res = (const T *) sm_at (bsm, S.off_res);
+  const T axc = (T) L.alpha[0].c, ayc = (T) L.alpha[1].c, azc = (T) L.alpha[2].c, lamc = (T) L.lambda.c;
+  const T D2 = (T) L.Delta*(T) L.Delta;
+  T * da = (T *) sm_at (bsm, S.off_da);
+  /* the mixed form's weights only in two dimensions (as its larger levels
+     relax); a 2D FP32 level is the mixed form's */
+  constexpr bool E32 = DIM == 3;
+  if (sizeof (T) == 8 && (DIM == 3 || !L.fast))
+    bot_sweeps_own<DIM, T, true> (S.gs, da, res, ax, ay, az, axc, ayc, azc, lam, lamc, D2, P.bc, P.nrelax, init);
+  else
+    bot_sweeps_own<DIM, T, E32> (S.gs, da, res, ax, ay, az, axc, ayc, azc, lam, lamc, D2, P.bc, P.nrelax, init);
 }
 
 template <int DIM>
@@ -2236,19 +2356,25 @@ __global__ void __launch_bounds__ (BOT_THREADS, 1) k_bottom (const __grid_consta
     const BotLevel & L = P.lv[m];
     const BotStage & S = P.sm[m];
     void * da = sm_at (bsm, S.off_da);
+    const void * al[3];
+    for (int d = 0; d < 3; d++) al[d] = d < DIM ? sm_at (bsm, S.off_alpha[d]) : NULL;
+    const void * res = sm_at (bsm, S.off_res);
+    const void * lam = sm_at (bsm, S.off_lambda);
+    const bmg_geom gs = S.gs;
+    if (DIM > 1 && gs.n >= 2 && (1 << (DIM*(31 - __clz (gs.n)))) <= 2*BOT_THREADS) {
+      if (L.st == BMG_ST_F64) bot_own_level<DIM, double> (P, m, bsm);
+      else bot_own_level<DIM, float> (P, m, bsm);
+      __syncthreads ();
+      continue;
+    }
     if (m == 0)
       bot_prolong_st<DIM> (L.st, S.gs, NULL, L.st, S.gs, da, P.bc, 1);
     else
       bot_prolong_st<DIM> (P.lv[m - 1].st, P.sm[m - 1].gs, sm_at (bsm, P.sm[m - 1].off_da),
                            L.st, S.gs, da, P.bc, 0);
     __syncthreads ();
-    const void * al[3];
-    for (int d = 0; d < 3; d++) al[d] = d < DIM ? sm_at (bsm, S.off_alpha[d]) : NULL;
-    const void * res = sm_at (bsm, S.off_res);
-    const void * lam = sm_at (bsm, S.off_lambda);
     /* levels of at most BOT_WARP_CELLS cells are relaxed by warp 0 alone,
        with warp barriers; the other warps wait at the level's end */
-    const bmg_geom gs = S.gs;
     const bool small = gs.size <= BOT_WARP_CELLS;
     const int nt = small ? 32 : blockDim.x, nrelax = P.nrelax, st = L.st;
     if (DIM == 2 && (al[0] == NULL) == (al[1] == NULL)) {
