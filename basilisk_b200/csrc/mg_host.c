@@ -681,40 +681,52 @@ static int resolve_coefs (bmg_grid * g, bmg_vector alpha, bmg_scalar lambda, coe
 /* restriction ({alpha, lambda}) (poisson.h:418-420) */
 static int restrict_coefs (bmg_grid * g, const coefs_t * c)
 {
+  /* (a constant component next to stored ones has no levels to restrict) */
+  int tail = 0;
+  double * f[BMG_MAXLEVEL + 1][3];
+  memset (f, 0, sizeof f);
+  for (int l = 0; l <= g->depth; l++)
+    for (int d = 0; d < g->dim; d++) f[l][d] = (double *) c->alpha64[l][d].p;
+  if (c->alpha_stored) {
+    int stored = 1;
+    for (int d = 0; d < g->dim; d++) stored = stored && f[0][d];
+    if (stored) tail = g->depth < bmg_restrict_face_tail_top () ? g->depth : bmg_restrict_face_tail_top ();
+  }
   for (int l = g->depth - 1; l >= 0; l--) {
-    if (c->alpha_stored) {
-      const double * fine[3] = {0, 0, 0};
-      double * coarse[3] = {0, 0, 0};
-      for (int d = 0; d < g->dim; d++) {
-        fine[d] = (const double *) c->alpha64[l + 1][d].p;
-        coarse[d] = (double *) c->alpha64[l][d].p;
-      }
-      CL (bmg_launch_restrict_face (g->dim, g->g64[l + 1], g->g64[l], fine, coarse,
-                                    level0_periodic (g, l), g->stream));
+    if (c->alpha_stored && l >= tail) {
+      const double * fine[3] = {f[l + 1][0], f[l + 1][1], f[l + 1][2]};
+      CL (bmg_launch_restrict_face (g->dim, g->g64[l + 1], g->g64[l], fine, f[l], level0_periodic (g, l),
+                                    g->stream));
     }
     if (c->lambda_stored)
       CL (bmg_launch_restrict (g->dim, BMG_ST_F64, BMG_ST_F64, g->g64[l + 1], g->g64[l],
                                c->lambda64[l + 1].p, (void *) c->lambda64[l].p, g->stream));
   }
+  if (tail > 0)
+    CL (bmg_launch_restrict_face_tail (g->dim, tail, g->g64, (double * const (*)[3]) f,
+                                       level0_periodic (g, 0), g->stream));
   return BMG_OK;
 }
 
 /* FP32 copies of the coefficients for the inner cycles of the mixed form */
 static int convert_coefs (bmg_grid * g, coefs_t * c)
 {
-  for (int l = 0; l <= g->depth; l++) {
+  bmg_convert jobs[4*(BMG_MAXLEVEL + 1)];
+  int n = 0;
+  for (int l = g->depth; l >= 0; l--) {
     for (int d = 0; d < g->dim; d++)
       if (c->alpha64[l][d].p) {
         float * dst = ws32 (g, W32_AX + d, l);
-        CL (bmg_launch_convert (g->dim, g->g64[l], g->g32[l], d, c->alpha64[l][d].p, dst, g->stream));
+        jobs[n++] = (bmg_convert) {(const double *) c->alpha64[l][d].p, dst, l, d};
         c->alpha32[l][d].p = dst;
       }
     if (c->lambda64[l].p) {
       float * dst = ws32 (g, W32_LAMBDA, l);
-      CL (bmg_launch_convert (g->dim, g->g64[l], g->g32[l], -1, c->lambda64[l].p, dst, g->stream));
+      jobs[n++] = (bmg_convert) {(const double *) c->lambda64[l].p, dst, l, -1};
       c->lambda32[l].p = dst;
     }
   }
+  if (n) CL (bmg_launch_convert (g->dim, n, jobs, g->g64, g->g32, g->depth, g->stream));
   return BMG_OK;
 }
 
@@ -1137,8 +1149,6 @@ static int solve (bmg_grid * g, field_t * a, field_t * b, coefs_t * c, int nrela
   /* sum of the r.h.s. (poisson.h:162-167) */
   CL (bmg_launch_sum (g->dim, g->g64[L], b->lv[L], g->d_partials, g->npartials, g->d_sum, g->stream));
   CK (cudaMemcpyAsync (g->h_pinned + 1, g->d_sum, sizeof (double), cudaMemcpyDeviceToHost, g->stream));
-  CK (cudaStreamSynchronize (g->stream));
-  s.sum = g->h_pinned[1];
   s.nrelax = nrelax > 0 ? nrelax : 4;
 
   /* mixed form, singular problem: FP64 zero-mean projection of b */
@@ -1154,6 +1164,7 @@ static int solve (bmg_grid * g, field_t * a, field_t * b, coefs_t * c, int nrela
   work_t w0 = {0., 0, 0, 0., 0};
   r = residual_tail (g, a, bdata, c, &lv, &s.resb, 1, &w0);
   if (r) return r;
+  s.sum = g->h_pinned[1];             /* (read back before the residual's maximum) */
   resb = s.resa = s.resb;
   if (tolerance == 0.)
     tolerance = TOLERANCE;

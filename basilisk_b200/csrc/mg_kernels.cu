@@ -49,6 +49,8 @@ template <int DIM, typename T, int MODE>
 __global__ void k_relax (bmg_geom g, T * out, const T * in, const T * __restrict__ rhs,
                          Coef<T> ax, Coef<T> ay, Coef<T> az, Coef<T> lam, T Delta, BCH bc)
 {
+  pdl_wait ();
+  pdl_trigger ();
   int i, j, k;
   if (!cell_of_thread<DIM> (g.n, i, j, k)) return;
   if (MODE != BMG_SWEEP_JACOBI && ((i + j + k) & 1) != MODE) return;
@@ -75,6 +77,8 @@ __global__ void k_relax3_pair (bmg_geom g, T * out, const T * in, const T * __re
                                double * acor, bmg_geom ga, bmg_bcdesc abc)
 {
   typedef typename std::conditional<sizeof (T) == 8, double2, float2>::type T2;
+  pdl_wait ();
+  pdl_trigger ();
   const int q = blockIdx.x*blockDim.x + threadIdx.x;
   const int j = blockIdx.y*blockDim.y + threadIdx.y;
   const int i = blockIdx.z*blockDim.z + threadIdx.z;
@@ -280,6 +284,10 @@ __global__ void k_restrict (bmg_geom gf, bmg_geom gc, const TF * __restrict__ f,
   c[cidx<DIM> (gc, i, j, k)] = sum/TC(1 << DIM);
 }
 
+/* the finest level of k_restrict_face_tail: 32 cells per side (the levels
+   below have at most 256, 4096 in 3D at 16) */
+#define FACE_TAIL_TOP 5
+
 struct FacePtrs {
   const double * f[3];
   double * c[3];
@@ -289,15 +297,14 @@ struct FacePtrs {
    rotation of the fine() offsets; every coarse cell writes its lower face,
    the last cell along each axis also its upper face. */
 template <int DIM>
-__global__ void k_restrict_face (bmg_geom gf, bmg_geom gc, FacePtrs p, int level0p)
+__device__ __forceinline__ void restrict_face_cell (const bmg_geom & gf, const bmg_geom & gc, const double * const * pf,
+                                                    double * const * pc, int level0p, int i, int j, int k)
 {
-  int i, j, k;
-  if (!cell_of_thread<DIM> (gc.n, i, j, k)) return;
   const int n = gc.n;
 #define FV(o0, o1, o2) f[cidx<DIM> (gf, 2*i + (o0), DIM > 1 ? 2*j + (o1) : 0, DIM > 2 ? 2*k + (o2) : 0)]
   for (int e = 0; e < DIM; e++) {
-    const double * f = p.f[e];
-    double * c = p.c[e];
+    const double * f = pf[e];
+    double * c = pc[e];
     const int ce = e == 0 ? i : e == 1 ? j : k;
     for (int side = 0; side < 2; side++) {
       if (side == 1 && ce != n - 1) break;
@@ -325,6 +332,41 @@ __global__ void k_restrict_face (bmg_geom gf, bmg_geom gc, FacePtrs p, int level
     }
   }
 #undef FV
+}
+
+template <int DIM>
+__global__ void k_restrict_face (bmg_geom gf, bmg_geom gc, FacePtrs p, int level0p)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  int i, j, k;
+  if (!cell_of_thread<DIM> (gc.n, i, j, k)) return;
+  restrict_face_cell<DIM> (gf, gc, p.f, p.c, level0p, i, j, k);
+}
+
+/* the levels from 2^(top - 1) cells per side down to one, each from the one
+   above, in one CTA: a barrier between levels instead of a launch (3 us
+   each) */
+struct FaceTail {
+  bmg_geom g[FACE_TAIL_TOP + 1];
+  double * f[FACE_TAIL_TOP + 1][3];
+  int top, level0p;
+};
+
+template <int DIM>
+__global__ void __launch_bounds__ (1024, 1) k_restrict_face_tail (const __grid_constant__ FaceTail P)
+{
+  pdl_wait ();
+  pdl_trigger ();
+  for (int l = P.top - 1; l >= 0; l--) {
+    const int m = (1 << l) - 1;
+    const double * fine[3] = {P.f[l + 1][0], P.f[l + 1][1], P.f[l + 1][2]};
+    for (int q = threadIdx.x; q < 1 << (DIM*l); q += blockDim.x) {
+      const int i = q >> ((DIM - 1)*l), j = DIM == 1 ? 0 : DIM == 2 ? q & m : (q >> l) & m;
+      restrict_face_cell<DIM> (P.g[l + 1], P.g[l], fine, P.f[l], l == 0 && P.level0p, i, j, DIM == 3 ? q & m : 0);
+    }
+    __syncthreads ();
+  }
 }
 
 /* ---------------------------------------------------------------- */
@@ -692,22 +734,46 @@ __global__ void k_unpack (bmg_geom g, int ni, int nj, int nk, int len, const dou
   }
 }
 
+/* FP32 copies of fields on all levels in one launch: job q (a level of a
+   field, extents ni x nj x nk, rows of len) has the blocks
+   first[q] .. first[q + 1] of blockIdx.x.  One launch for what took one per
+   level and component (28 of them for a 64^3 solve with lambda stored). */
+#define CONVERT_JOBS 64
+struct ConvertJobs {
+  const double * src[CONVERT_JOBS];
+  float * dst[CONVERT_JOBS];
+  int first[CONVERT_JOBS + 1];
+  unsigned char level[CONVERT_JOBS];
+  signed char face[CONVERT_JOBS];
+  bmg_geom g64[BMG_MAXLEVEL + 1], g32[BMG_MAXLEVEL + 1];
+  int n;
+};
+
 template <int DIM>
-__global__ void k_convert (bmg_geom g64, bmg_geom g32, int ni, int nj, int nk, int len,
-                           const double * __restrict__ src, float * __restrict__ dst)
+__global__ void k_convert (const __grid_constant__ ConvertJobs J)
 {
-  const Row<DIM> r (ni, nj);
-  if (!r.ok) return;
-  double v[ROWU];
+  int q = 0;
+  while ((int) blockIdx.x >= J.first[q + 1]) q++;
+  const bmg_geom & g64 = J.g64[J.level[q]], & g32 = J.g32[J.level[q]];
+  const int n = g64.n, f = J.face[q];
+  const int ni = n + (f == 0), nj = DIM > 1 ? n + (f == 1) : 1, nk = DIM > 2 ? n + (f == 2) : 1;
+  const int len = DIM == 1 ? ni : DIM == 2 ? nj : nk, rows = DIM == 1 ? 1 : DIM == 2 ? ni : ni*nj;
+  const double * src = J.src[q];
+  float * dst = J.dst[q];
+  /* a warp takes a row, 256 elements at a time */
+  const int row = (blockIdx.x - J.first[q])*(blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int i = DIM == 1 ? 0 : DIM == 2 ? row : row/nj, j = DIM == 3 ? row - i*nj : 0;
+  const long long s0 = DIM == 1 ? cidx<1> (g64, 0, 0, 0) : DIM == 2 ? cidx<2> (g64, i, 0, 0) : cidx<3> (g64, i, j, 0);
+  const long long d0 = DIM == 1 ? cidx<1> (g32, 0, 0, 0) : DIM == 2 ? cidx<2> (g32, i, 0, 0) : cidx<3> (g32, i, j, 0);
+  for (int k0 = lane; k0 < len; k0 += 256) {
+    double v[8];
 #pragma unroll
-  for (int u = 0; u < ROWU; u++) {
-    const int k = r.first + u*blockDim.x;
-    if (k < len) v[u] = src[r.padded (g64, k)];
-  }
+    for (int u = 0; u < 8; u++)
+      if (k0 + 32*u < len) v[u] = src[s0 + k0 + 32*u];
 #pragma unroll
-  for (int u = 0; u < ROWU; u++) {
-    const int k = r.first + u*blockDim.x;
-    if (k < len) dst[r.padded (g32, k)] = (float) v[u];
+    for (int u = 0; u < 8; u++)
+      if (k0 + 32*u < len) dst[d0 + k0 + 32*u] = (float) v[u];
   }
 }
 
@@ -776,22 +842,22 @@ void relax_dim (int mode, bmg_geom g, void * out, const void * in, const void * 
     bmg_bcdesc none;
     memset (&none, 0, sizeof none);
     if (mode == BMG_SWEEP_RED)
-      k_relax3_pair<T, BMG_SWEEP_RED, false><<<gb, bb, 0, s>>> (
+      pdl_launch (k_relax3_pair<T, BMG_SWEEP_RED, false>, gb, bb, 0, s, 
         g, (T *) out, (const T *) in, (const T *) rhs, ax, ay, az, lam, (T) Delta, h, NULL, g, none);
     else
-      k_relax3_pair<T, BMG_SWEEP_BLACK, false><<<gb, bb, 0, s>>> (
+      pdl_launch (k_relax3_pair<T, BMG_SWEEP_BLACK, false>, gb, bb, 0, s, 
         g, (T *) out, (const T *) in, (const T *) rhs, ax, ay, az, lam, (T) Delta, h, NULL, g, none);
     return;
   }
   dim3 gb = grid_shape<DIM> (g.n), bb = block_shape<DIM> ();
   if (mode == BMG_SWEEP_JACOBI)
-    k_relax<DIM, T, BMG_SWEEP_JACOBI><<<gb, bb, 0, s>>> (g, (T *) out, (const T *) in,
+    pdl_launch (k_relax<DIM, T, BMG_SWEEP_JACOBI>, gb, bb, 0, s, g, (T *) out, (const T *) in,
                                                           (const T *) rhs, ax, ay, az, lam, (T) Delta, h);
   else if (mode == BMG_SWEEP_RED)
-    k_relax<DIM, T, BMG_SWEEP_RED><<<gb, bb, 0, s>>> (g, (T *) out, (const T *) in,
+    pdl_launch (k_relax<DIM, T, BMG_SWEEP_RED>, gb, bb, 0, s, g, (T *) out, (const T *) in,
                                                        (const T *) rhs, ax, ay, az, lam, (T) Delta, h);
   else
-    k_relax<DIM, T, BMG_SWEEP_BLACK><<<gb, bb, 0, s>>> (g, (T *) out, (const T *) in,
+    pdl_launch (k_relax<DIM, T, BMG_SWEEP_BLACK>, gb, bb, 0, s, g, (T *) out, (const T *) in,
                                                          (const T *) rhs, ax, ay, az, lam, (T) Delta, h);
 }
 
@@ -867,7 +933,7 @@ void restrict_dim (int stf, int stc, bmg_geom gf, bmg_geom gc, const void * f, v
 template <int DIM>
 void restrict_face_dim (bmg_geom gf, bmg_geom gc, FacePtrs p, int level0p, cudaStream_t s)
 {
-  k_restrict_face<DIM><<<grid_shape<DIM> (gc.n), block_shape<DIM> (), 0, s>>> (gf, gc, p, level0p);
+  pdl_launch (k_restrict_face<DIM>, grid_shape<DIM> (gc.n), block_shape<DIM> (), 0, s, gf, gc, p, level0p);
 }
 
 template <int DIM>
@@ -983,17 +1049,6 @@ void unpack_dim (bmg_geom g, int face_dim, const double * p, double * c, cudaStr
   extents<DIM> (g.n, face_dim, ni, nj, nk);
   row_launch<DIM> (ni, nj, nk, len, gb, bb);
   k_unpack<DIM><<<gb, bb, 0, s>>> (g, ni, nj, nk, len, p, c);
-}
-
-template <int DIM>
-void convert_dim (bmg_geom g64, bmg_geom g32, int face_dim, const double * src, float * dst,
-                  cudaStream_t s)
-{
-  int ni, nj, nk, len;
-  dim3 gb, bb;
-  extents<DIM> (g64.n, face_dim, ni, nj, nk);
-  row_launch<DIM> (ni, nj, nk, len, gb, bb);
-  k_convert<DIM><<<gb, bb, 0, s>>> (g64, g32, ni, nj, nk, len, src, dst);
 }
 
 /* the rows of a compact face array of direction e */
@@ -1304,6 +1359,25 @@ int bmg_launch_restrict_face (int dim, bmg_geom gf, bmg_geom gc, const double * 
   return status_of_launch ();
 }
 
+int bmg_restrict_face_tail_top (void) { return FACE_TAIL_TOP; }
+
+int bmg_launch_restrict_face_tail (int dim, int top, const bmg_geom * g, double * const (* f)[3], int level0p,
+                                   cudaStream_t s)
+{
+  if (top < 1 || top > FACE_TAIL_TOP) return (int) cudaErrorInvalidValue;
+  FaceTail P;
+  memset (&P, 0, sizeof P);
+  for (int l = 0; l <= top; l++) {
+    P.g[l] = g[l];
+    for (int e = 0; e < dim; e++) P.f[l][e] = f[l][e];
+  }
+  P.top = top; P.level0p = level0p;
+  if (dim == 1) pdl_launch (k_restrict_face_tail<1>, dim3 (1), dim3 (1024), 0, s, P);
+  else if (dim == 2) pdl_launch (k_restrict_face_tail<2>, dim3 (1), dim3 (1024), 0, s, P);
+  else pdl_launch (k_restrict_face_tail<3>, dim3 (1), dim3 (1024), 0, s, P);
+  return status_of_launch ();
+}
+
 int bmg_launch_residual (int dim, int st_res, bmg_geom g, bmg_geom gres, const double * a,
                          const double * b, const bmg_coef * alpha, bmg_coef lambda,
                          double Delta, void * res, unsigned long long * maxres,
@@ -1360,12 +1434,12 @@ int bmg_launch_relax_correct3d (int st, bmg_geom g, void * out, const void * in,
   BCH h = bch_of (bc);
   const dim3 bb (32, 4, 2), gb ((g.n/2 + 31)/32, (g.n + 3)/4, (g.n + 1)/2);
   if (st == BMG_ST_F64)
-    k_relax3_pair<double, BMG_SWEEP_BLACK, true><<<gb, bb, 0, s>>> (
+    pdl_launch (k_relax3_pair<double, BMG_SWEEP_BLACK, true>, gb, bb, 0, s, 
       g, (double *) out, (const double *) in, (const double *) rhs, coef_of<double> (alpha[0]),
       coef_of<double> (alpha[1]), coef_of<double> (alpha[2]), coef_of<double> (lambda),
       Delta, h, acor, ga, *abc);
   else
-    k_relax3_pair<float, BMG_SWEEP_BLACK, true><<<gb, bb, 0, s>>> (
+    pdl_launch (k_relax3_pair<float, BMG_SWEEP_BLACK, true>, gb, bb, 0, s, 
       g, (float *) out, (const float *) in, (const float *) rhs, coef_of<float> (alpha[0]),
       coef_of<float> (alpha[1]), coef_of<float> (alpha[2]), coef_of<float> (lambda),
       (float) Delta, h, acor, ga, *abc);
@@ -1418,11 +1492,34 @@ int bmg_launch_unpack (int dim, bmg_geom g, int face_dim, const double * padded,
   return status_of_launch ();
 }
 
-int bmg_launch_convert (int dim, bmg_geom g64, bmg_geom g32, int face_dim, const double * src,
-                        float * dst, cudaStream_t s)
+int bmg_launch_convert (int dim, int njobs, const bmg_convert * jobs, const bmg_geom * g64,
+                        const bmg_geom * g32, int depth, cudaStream_t s)
 {
-  DISPATCH_DIM (dim, convert_dim, g64, g32, face_dim, src, dst, s);
-  return status_of_launch ();
+  for (int q0 = 0; q0 < njobs; q0 += CONVERT_JOBS) {
+    ConvertJobs J;
+    memset (&J, 0, sizeof J);
+    J.n = njobs - q0 < CONVERT_JOBS ? njobs - q0 : CONVERT_JOBS;
+    for (int l = 0; l <= depth; l++) { J.g64[l] = g64[l]; J.g32[l] = g32[l]; }
+    long long blocks = 0;
+    for (int q = 0; q < J.n; q++) {
+      const bmg_convert & c = jobs[q0 + q];
+      int ni, nj, nk;
+      if (dim == 1) extents<1> (g64[c.level].n, c.face_dim, ni, nj, nk);
+      else if (dim == 2) extents<2> (g64[c.level].n, c.face_dim, ni, nj, nk);
+      else extents<3> (g64[c.level].n, c.face_dim, ni, nj, nk);
+      J.src[q] = c.src; J.dst[q] = c.dst;
+      J.level[q] = (unsigned char) c.level; J.face[q] = (signed char) c.face_dim;
+      J.first[q] = (int) blocks;
+      blocks += ((dim == 1 ? 1 : dim == 2 ? ni : (long long) ni*nj) + 7)/8;
+      J.first[q + 1] = (int) blocks;
+    }
+    if (dim == 1) k_convert<1><<<(int) blocks, 256, 0, s>>> (J);
+    else if (dim == 2) k_convert<2><<<(int) blocks, 256, 0, s>>> (J);
+    else k_convert<3><<<(int) blocks, 256, 0, s>>> (J);
+    const int e = status_of_launch ();
+    if (e) return e;
+  }
+  return 0;
 }
 
 int bmg_launch_fill (int dim, int st, bmg_geom g, void * f, double v, cudaStream_t s)

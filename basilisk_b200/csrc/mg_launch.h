@@ -74,6 +74,12 @@ int bmg_launch_restrict_face (int dim, bmg_geom gf, bmg_geom gc,
                               const double * const * fine, double * const * coarse,
                               int level0p, cudaStream_t s);
 
+/* the levels top - 1 .. 0, each from the one above, in one launch (top at
+   most bmg_restrict_face_tail_top ()); arrays by level */
+int bmg_restrict_face_tail_top (void);
+int bmg_launch_restrict_face_tail (int dim, int top, const bmg_geom * g, double * const (* f)[3], int level0p,
+                                   cudaStream_t s);
+
 int bmg_launch_residual (int dim, int st_res, bmg_geom g, bmg_geom gres,
                          const double * a, const double * b,
                          const bmg_coef * alpha, bmg_coef lambda, double Delta,
@@ -124,8 +130,10 @@ int bmg_launch_pack (int dim, int st, bmg_geom g, int face_dim,
 int bmg_launch_unpack (int dim, bmg_geom g, int face_dim, const double * padded,
                        double * compact, cudaStream_t s);
 
-int bmg_launch_convert (int dim, bmg_geom g64, bmg_geom g32, int face_dim,
-                        const double * src, float * dst, cudaStream_t s);
+/* FP32 copies of level arrays of fields, all jobs in one launch */
+typedef struct { const double * src; float * dst; int level, face_dim; } bmg_convert;
+int bmg_launch_convert (int dim, int njobs, const bmg_convert * jobs, const bmg_geom * g64,
+                        const bmg_geom * g32, int depth, cudaStream_t s);
 
 int bmg_launch_fill (int dim, int st, bmg_geom g, void * f, double v, cudaStream_t s);
 
