@@ -316,15 +316,264 @@ __global__ void __launch_bounds__ (1024, 1) k_blocks_bottom (const __grid_consta
   }
 }
 
-#define NT 256
+/* ---------------------------------------------------------------- */
+/* the same levels as one grid in shared memory                      */
+/* ---------------------------------------------------------------- */
 
-dim3 grid_of (long long threads, int m) { return dim3 ((unsigned) ((threads + NT - 1)/NT), m, 1); }
+#define ST_THREADS 1024
+/* the shared memory of one CTA */
+#define ST_BYTES (227*1024)
+
+struct StagedParams {
+  BottomParams bot;
+  int dims[3], periodic[3];       /* of the decomposition */
+  unsigned off_c, off_w, off_nb;  /* shared memory: coarser iterate, weights, neighbours */
+};
+
+/* a level of the blocks as one grid, its cells split by colour: extents,
+   half the cells, half a row */
+template <int DIM>
+struct Joint {
+  int l, N[3], half, nh;
+  __device__ __forceinline__ Joint (const StagedParams & P, int level) : l (level)
+  {
+    half = 1;
+#pragma unroll
+    for (int e = 0; e < 3; e++) { N[e] = e < DIM ? P.dims[e] << l : 1; half *= N[e]; }
+    half >>= 1;
+    nh = N[DIM - 1] >> 1;
+  }
+  __device__ __forceinline__ int slot (const int * x) const
+  {
+    const int row = DIM == 1 ? 0 : DIM == 2 ? x[0] : x[0]*N[1] + x[1];
+    const int c = (x[0] + (DIM > 1 ? x[1] : 0) + (DIM > 2 ? x[2] : 0)) & 1;
+    return c*half + row*nh + (x[DIM - 1] >> 1);
+  }
+  /* cell q of colour c */
+  __device__ __forceinline__ void cell (int c, int q, int * x) const
+  {
+    const int row = q/nh, h = q - row*nh;
+    x[0] = x[1] = x[2] = 0;
+    if (DIM == 2) x[0] = row;
+    if (DIM == 3) { x[0] = row/N[1]; x[1] = row - x[0]*N[1]; }
+    x[DIM - 1] = 2*h + ((c + x[0] + x[1]) & 1);
+  }
+  __device__ __forceinline__ int block (const StagedParams & P, const int * x) const
+  {
+    return ((x[0] >> l)*P.dims[1] + (DIM > 1 ? x[1] >> l : 0))*P.dims[2] + (DIM > 2 ? x[2] >> l : 0);
+  }
+  /* iterate u at a cell, or at a position beyond the sides: the image of
+     the cell it mirrors, with its block's conditions */
+  __device__ __forceinline__ double at (const StagedParams & P, const double * u, int i, int j, int k) const
+  {
+    int x[3] = {i, j, k}, side[3];
+    bool box = false;
+#pragma unroll
+    for (int e = 0; e < DIM; e++) {
+      side[e] = -1;
+      if (x[e] >= 0 && x[e] < N[e]) continue;
+      const bool lo = x[e] < 0;
+      if (P.periodic[e]) x[e] = lo ? N[e] - 1 : 0;
+      else { x[e] = lo ? 0 : N[e] - 1; side[e] = 2*e + lo; box = true; }
+    }
+    double v = u[slot (x)];
+    if (box) {
+      const bmg_bcdesc & bc = P.bot.B.blk[block (P, x)].bc;
+#pragma unroll
+      for (int e = 0; e < DIM; e++)
+        if (side[e] >= 0 && bc.type[side[e]] == 1 /* BMG_DIRICHLET */) v = v*(-1.);
+    }
+    return v;
+  }
+};
+
+/* the prolongation of level l - 1 (k_prolong's expression and order) at a
+   cell of level l */
+template <int DIM>
+__device__ __forceinline__ double staged_bilinear (const StagedParams & P, const Joint<DIM> & C,
+                                                   const double * s, const int * x)
+{
+  const int pi = x[0] >> 1, cx = (x[0] & 1) ? 1 : -1, pj = x[1] >> 1, cy = (x[1] & 1) ? 1 : -1;
+  const int pk = x[2] >> 1, cz = (x[2] & 1) ? 1 : -1;
+  auto a = [&] (int i, int j, int k) { return C.at (P, s, i, j, k); };
+  if (DIM == 1) return (3.*a (pi, 0, 0) + a (pi + cx, 0, 0))/4.;
+  if (DIM == 2)
+    return (9.*a (pi, pj, 0) + 3.*(a (pi + cx, pj, 0) + a (pi, pj + cy, 0)) + a (pi + cx, pj + cy, 0))/16.;
+  return (27.*a (pi, pj, pk) + 9.*(a (pi + cx, pj, pk) + a (pi, pj + cy, pk) + a (pi, pj, pk + cz)) +
+          3.*(a (pi + cx, pj + cy, pk) + a (pi + cx, pj, pk + cz) + a (pi, pj + cy, pk + cz)) +
+          a (pi + cx, pj + cy, pk + cz))/64.;
+}
+
+/* zero or prolongation, then the sweeps of one level: u its iterate, c that
+   of the level below.  A thread owns NS cells of each colour.  The image of
+   a box side is read only by the cell it mirrors, whose weight takes its
+   sign and whose neighbour there is the cell itself.  Weights and
+   neighbours stay in registers when NS = 1, in shared memory (the thread's
+   own words) otherwise. */
+template <int DIM, int NS>
+__device__ __noinline__ void staged_level (const StagedParams & P, int l)
+{
+  extern __shared__ __align__ (16) unsigned char ssm[];
+  const bool even = (P.bot.hi - l) & 1;
+  double * u = (double *) (ssm + (even ? P.off_c : 0));
+  const double * uc = (const double *) (ssm + (even ? 0 : P.off_c));
+  double * W = (double *) (ssm + P.off_w);
+  ushort2 * NB = (ushort2 *) (ssm + P.off_nb);
+  const Joint<DIM> G (P, l), C (P, l > 0 ? l - 1 : 0);
+  const int tid = threadIdx.x, half = G.half, cells = 2*half;
+  const int active = half < ST_THREADS ? (half + 31) & ~31 : ST_THREADS;
+  const double D2 = P.bot.Delta[l]*P.bot.Delta[l];
+  double w[2][2*DIM], be[2][NS], d[2][NS], y[2][NS];
+  int nb[2][2*DIM];
+  bool plain = false;             /* a diagonal outside exact_quotient's range */
+#pragma unroll
+  for (int c = 0; c < 2; c++)
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+      const int q = tid + s*ST_THREADS;
+      if (q >= half) continue;
+      int x[3];
+      G.cell (c, q, x);
+      const int b = G.block (P, x), p = c*half + q, m = (1 << l) - 1;
+      const bmg_blk_level & L = P.bot.B.lv[(long long) l*P.bot.B.nb + b];
+      const bmg_geom & g = P.bot.g[l];
+      const long long id = cidx<DIM> (g, x[0] & m, x[1] & m, x[2] & m);
+      be[c][s] = (-D2)*L.res[id];
+      double dd = (-coef_of<double> (L.lambda).at (id))*D2;
+#pragma unroll
+      for (int e = 0; e < DIM; e++) {
+        const Coef<double> al = coef_of<double> (L.alpha[e]);
+        const double w1 = al.at (id + cstride<DIM> (g, e)), w0 = al.at (id);
+        dd += w1 + w0;
+        double wv[2];
+        int at[2];
+#pragma unroll
+        for (int lo = 0; lo < 2; lo++) {
+          const bool edge = x[e] == (lo ? 0 : G.N[e] - 1), box = edge && !P.periodic[e];
+          const double v = lo ? w0 : w1;
+          wv[lo] = box && P.bot.B.blk[b].bc.type[2*e + lo] == 1 ? -v : v;
+          int z[3] = {x[0], x[1], x[2]};
+          z[e] = edge ? (lo ? G.N[e] - 1 : 0) : x[e] + (lo ? -1 : 1);
+          at[lo] = box ? p : G.slot (z);
+        }
+        if (NS == 1) {
+          w[c][2*e] = wv[0]; w[c][2*e + 1] = wv[1];
+          nb[c][2*e] = at[0]; nb[c][2*e + 1] = at[1];
+        }
+        else {
+          W[2*e*cells + p] = wv[0]; W[(2*e + 1)*cells + p] = wv[1];
+          NB[e*cells + p] = make_ushort2 (at[0], at[1]);
+        }
+      }
+      d[c][s] = dd;
+      y[c][s] = 1./dd;
+      plain = plain || divisor_unsafe (dd);
+      u[p] = l == P.bot.lo ? 0. : staged_bilinear<DIM> (P, C, uc, x);
+    }
+  __syncthreads ();
+  if (tid < active)
+    for (int sw = 0; sw < P.bot.nrelax; sw++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+          const int q = tid + s*ST_THREADS, p = c*half + q;
+          if (q >= half) continue;
+          double m = be[c][s];
+#pragma unroll
+          for (int e = 0; e < DIM; e++)
+            if (NS == 1) m = m + (w[c][2*e]*u[nb[c][2*e]] + w[c][2*e + 1]*u[nb[c][2*e + 1]]);
+            else {
+              const ushort2 at = NB[e*cells + p];
+              m = m + (W[2*e*cells + p]*u[at.x] + W[(2*e + 1)*cells + p]*u[at.y]);
+            }
+          double v = exact_quotient (m, d[c][s], y[c][s]);
+          if (__any_sync (__activemask (), plain || quotient_unsafe (m))) v = m/d[c][s];
+          u[p] = v;
+        }
+        asm volatile ("bar.sync 1, %0;" :: "r" (active) : "memory");
+      }
+  __syncthreads ();
+}
+
+/* k_blocks_bottom's levels with the blocks joined into one grid (they are
+   one: a block's ghosts are its neighbours' cells): the iterate split by
+   colour in shared memory, one copy of a cell instead of its images, the
+   coefficients read once per level, quotients through the diagonal's
+   reciprocal.  Only level hi's iterate goes back to the blocks, with all
+   its images.  The residual is restricted in the blocks' arrays.  Bound:
+   the latency of a pass, and at 4096 cells its shared-memory accesses. */
+template <int DIM>
+__global__ void __launch_bounds__ (ST_THREADS, 1) k_blocks_staged (const __grid_constant__ StagedParams P)
+{
+  extern __shared__ __align__ (16) unsigned char ssm[];
+  pdl_wait ();
+  pdl_trigger ();
+  const bmg_blocks & B = P.bot.B;
+  for (int l = P.bot.restrict_src ? P.bot.hi : P.bot.hi - 1; l >= P.bot.lo; l--) {
+    const int cells = 1 << (DIM*l);
+    for (int q = threadIdx.x; q < cells*B.m; q += blockDim.x) {
+      const bmg_blk_level * lv = B.lv + (long long) l*B.nb + (q >> (DIM*l));
+      int i, j, k;
+      cell_at<DIM> (q & (cells - 1), l, i, j, k);
+      lv->res[cidx<DIM> (P.bot.g[l], i, j, k)] = mean<DIM> (P.bot.g[l + 1], lv[B.nb].res, i, j, k);
+    }
+    __syncthreads ();
+  }
+  for (int l = P.bot.lo; l <= P.bot.hi; l++)
+    if (Joint<DIM> (P, l).half <= ST_THREADS) staged_level<DIM, 1> (P, l);
+    else staged_level<DIM, 2> (P, l);
+  const int l = P.bot.hi, n = 1 << l, e = n + 2, cells = DIM == 1 ? e : DIM == 2 ? e*e : e*e*e;
+  const Joint<DIM> G (P, l);
+  const double * u = (const double *) ssm;
+  for (int q = threadIdx.x; q < cells*B.m; q += blockDim.x) {
+    const int b = q/cells, r = q - b*cells;
+    const int i = (DIM == 1 ? r : DIM == 2 ? r/e : r/(e*e)) - 1;
+    const int j = DIM == 1 ? 0 : (DIM == 2 ? r % e : r/e % e) - 1, k = DIM == 3 ? r % e - 1 : 0;
+    const int b0 = b/(P.dims[1]*P.dims[2]), b1 = b/P.dims[2] % P.dims[1], b2 = b % P.dims[2];
+    B.lv[(long long) l*B.nb + b].da[cidx<DIM> (P.bot.g[l], i, j, k)] =
+      G.at (P, u, (b0 << l) + i, (b1 << l) + j, (b2 << l) + k);
+  }
+}
 
 int status_of (cudaError_t launched)
 {
   const cudaError_t e = cudaGetLastError ();
   return launched != cudaSuccess ? (int) launched : (int) e;
 }
+
+/* the launch, or -1 when the levels don't fit the shared memory (three
+   dimensions above some 3300 cells) */
+template <int DIM>
+int staged_dim (const BottomParams & bot, const int * dims, const int * periodic, cudaStream_t s)
+{
+  long long cells = (long long) bot.B.nb << (DIM*bot.hi);
+  if (bot.B.m != bot.B.nb || cells > 4*ST_THREADS) return -1;
+  StagedParams P;
+  memset (&P, 0, sizeof P);
+  P.bot = bot;
+  for (int e = 0; e < 3; e++) { P.dims[e] = e < DIM ? dims[e] : 1; P.periodic[e] = e < DIM && periodic[e]; }
+  const bool words = cells > 2*ST_THREADS;
+  P.off_c = (unsigned) (cells*8);
+  P.off_w = P.off_c + (unsigned) (cells*8 >> DIM);
+  P.off_nb = P.off_w + (words ? (unsigned) (cells*2*DIM*8) : 0);
+  const unsigned bytes = P.off_nb + (words ? (unsigned) (cells*DIM*sizeof (ushort2)) : 0);
+  if (bytes > ST_BYTES) return -1;
+  static unsigned char configured[64];
+  int dev = 0;
+  cudaGetDevice (&dev);
+  if (dev < 0 || dev >= 64) return (int) cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute (k_blocks_staged<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_BYTES);
+    if (e != cudaSuccess) return (int) e;
+    configured[dev] = 1;
+  }
+  return status_of (pdl_launch (k_blocks_staged<DIM>, dim3 (1), dim3 (ST_THREADS), bytes, s, P));
+}
+
+#define NT 256
+
+dim3 grid_of (long long threads, int m) { return dim3 ((unsigned) ((threads + NT - 1)/NT), m, 1); }
 
 template <int DIM>
 cudaError_t relax_dim (int mode, int odd, bmg_geom g, int l, bmg_blocks B, double Delta, cudaStream_t s)
@@ -386,13 +635,17 @@ int bmg_blocks_residual (int dim, bmg_geom g, int l, bmg_blocks B, double Delta,
 }
 
 int bmg_blocks_bottom (int dim, const bmg_geom * g, const double * Delta, int lo, int hi,
-                       bmg_blocks B, int nrelax, int restrict_src, cudaStream_t s)
+                       bmg_blocks B, const int * dims, const int * periodic, int nrelax,
+                       int restrict_src, cudaStream_t s)
 {
   if (lo < 1 || hi < lo || hi > BMG_MAXLEVEL) return (int) cudaErrorInvalidValue;
   BottomParams P;
   memset (&P, 0, sizeof P);
   for (int l = lo; l <= hi + (restrict_src ? 1 : 0); l++) { P.g[l] = g[l]; P.Delta[l] = Delta[l]; }
   P.B = B; P.lo = lo; P.hi = hi; P.nrelax = nrelax; P.restrict_src = restrict_src;
+  const int r = dim == 1 ? staged_dim<1> (P, dims, periodic, s)
+    : dim == 2 ? staged_dim<2> (P, dims, periodic, s) : staged_dim<3> (P, dims, periodic, s);
+  if (r >= 0) return r;
   return status_of (dim == 1 ? pdl_launch (k_blocks_bottom<1>, dim3 (1), dim3 (1024), 0, s, P)
                     : dim == 2 ? pdl_launch (k_blocks_bottom<2>, dim3 (1), dim3 (1024), 0, s, P)
                     : pdl_launch (k_blocks_bottom<3>, dim3 (1), dim3 (1024), 0, s, P));

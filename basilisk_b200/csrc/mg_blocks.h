@@ -56,10 +56,12 @@ int bmg_blocks_residual (int dim, bmg_geom g, int l, bmg_blocks B, double Delta,
                          unsigned long long * maxres, cudaStream_t s);
 /* levels lo..hi of a cycle in one CTA, all blocks on its device: the
    restriction of res from level hi + 1 (when restrict_src), zero or
-   prolongation and nrelax red-black sweeps of each level */
+   prolongation and nrelax red-black sweeps of each level; dims, periodic:
+   of the decomposition */
 #define BMG_BLOCKS_CTA_CELLS 4096       /* cells of level hi, all blocks */
 int bmg_blocks_bottom (int dim, const bmg_geom * g, const double * Delta, int lo, int hi,
-                       bmg_blocks B, int nrelax, int restrict_src, cudaStream_t s);
+                       bmg_blocks B, const int * dims, const int * periodic, int nrelax,
+                       int restrict_src, cudaStream_t s);
 
 #ifdef __cplusplus
 }

@@ -569,7 +569,8 @@ static int shard_cycle (bmg_shard * s, blk_t * k, int nrelax, int minlevel, int 
   }
   int odd = 0;                        /* the iterate of the level below is in da2 */
   if (top >= minlevel) {
-    EACH (bmg_blocks_bottom (dim, g, Delta, minlevel, top, B, nrelax, top < L, s->stream[d]));
+    EACH (bmg_blocks_bottom (dim, g, Delta, minlevel, top, B, s->dims, s->periodic, nrelax, top < L,
+                             s->stream[d]));
     (*launches)++;
   }
   const bmg_geom none = {0};

@@ -169,3 +169,34 @@ def test_blocks_of_one_cell():
     A = np.array([[-6, 1, 1, 0], [1, -6, 0, 1], [1, 0, -6, 1], [0, 1, 1, -6]], float)
     np.testing.assert_allclose(a.get().ravel(), np.linalg.solve(A, b.ravel() / 4.0), atol=1e-10)
     sg.close()
+
+
+@pytest.mark.parametrize("relax", ["rbgs", "jacobi"])
+@pytest.mark.parametrize("dim,depth,dims", [(1, 4, (3,)), (2, 4, (3, 1)), (2, 5, (3, 1)), (2, 3, (5, 3)),
+                                            (3, 3, (3, 1, 1))])
+def test_repeated_blocks_equal_one_block(dim, depth, dims, relax):
+    """A periodic domain of equal blocks, their number not a power of two:
+    every block is the periodic solve of one block (the coarse levels of all
+    of them joined in one CTA)."""
+    import helpers
+    prob = helpers.random_problem(dim, depth, np.random.default_rng(50 + dim + depth),
+                                  periodic=tuple(range(dim)), lam="field")
+    for d, c in enumerate(prob["alpha"]):
+        c[(slice(None),) * d + (-1,)] = c[(slice(None),) * d + (0,)]
+    out = []
+    for D in ((1,) * dim, dims):
+        sg = ShardedGrid(dim, depth, dims=D, periodic=tuple(range(dim)), relax=relax, L0=float(D[0]))
+        faces = []
+        for d, c in enumerate(prob["alpha"]):
+            inner = np.tile(np.delete(c, -1, axis=d), D)
+            faces.append(np.concatenate([inner, np.take(inner, [0], axis=d)], axis=d))
+        a = sg.scalar()
+        a.set(np.zeros(np.tile(prob["b"], D).shape))
+        st = sg.poisson(a, sg.scalar(np.tile(prob["b"], D)), alpha=sg.face_vector(faces),
+                        lambda_=sg.scalar(np.tile(prob["lambda"], D)), tolerance=1e-8)
+        out.append((st, a.get()))
+        sg.close()
+    (s1, a1), (sn, an) = out
+    for key in ("i", "nrelax", "resb", "resa"):
+        assert sn[key] == s1[key], (key, sn, s1)
+    np.testing.assert_array_equal(an, np.tile(a1, dims))
