@@ -46,6 +46,21 @@ int bmg_blocks_relax (int dim, int mode, int odd, bmg_geom g, int l, bmg_blocks 
 /* zero (gc.n = 0) or bilinear prolongation of level l - 1 (whose iterate is
    in da2 when odd) into da of level l, with the same boundary */
 int bmg_blocks_prolong (int dim, int odd, bmg_geom gc, bmg_geom g, int l, bmg_blocks B, cudaStream_t s);
+/* two dimensions, l >= 1: nsweeps (at most BMG_BLOCKS_SWEEPS) red-black sweeps
+   of level l from `in' (da, da2, zero, or the prolongation of level l - 1's
+   da or da2) into `out' (da or da2; not `in'), with the images when images.
+   No launch of the same sweeps on another device writes what it reads */
+#define BMG_BLOCKS_SWEEPS 4
+/* the cells of a level on a device up to which four sweeps of tiles beat
+   eight passes: the window is three times the tile, which costs nothing
+   while the passes are bound by their launches (2 x 2 blocks, ms per cycle
+   with / without tiles on that level: 64^2 0.22 / 0.24, 128^2 0.23 / 0.25,
+   256^2 0.34 / 0.35, 512^2 0.83 / 0.78, 1024^2 2.59 / 2.32) */
+#define BMG_BLOCKS_TILE_CELLS (1 << 19)
+enum { BMG_BLOCKS_DA = 0, BMG_BLOCKS_DA2, BMG_BLOCKS_COARSE_DA, BMG_BLOCKS_COARSE_DA2, BMG_BLOCKS_ZERO };
+int bmg_blocks_tile (bmg_geom gc, bmg_geom g, int l, bmg_blocks B, const int * dims,
+                     const int * periodic, double Delta, int in, int out, int nsweeps, int images,
+                     cudaStream_t s);
 /* restriction of res from level l + 1 into level l */
 int bmg_blocks_restrict (int dim, bmg_geom gf, bmg_geom g, int l, bmg_blocks B, cudaStream_t s);
 /* a += da (da2 when odd) on the finest level, with the boundary of a */

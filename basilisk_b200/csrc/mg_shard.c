@@ -548,7 +548,8 @@ static int single_cell_sweep (bmg_shard * s, blk_t * k, long long * launches)
   return BMG_OK;
 }
 
-/* mg_cycle (poisson.h:32-90) over the blocks, one pass per launch with its
+/* mg_cycle (poisson.h:32-90) over the blocks: the coarse levels in one CTA,
+   several sweeps per launch on tiles, or one pass per launch with its
    boundary */
 static int shard_cycle (bmg_shard * s, blk_t * k, int nrelax, int minlevel, int maxlevel,
                         long long * launches)
@@ -568,6 +569,8 @@ static int shard_cycle (bmg_shard * s, blk_t * k, int nrelax, int minlevel, int 
     *launches += nd;
   }
   int odd = 0;                        /* the iterate of the level below is in da2 */
+  int most = 0;                       /* blocks of a device */
+  for (int d = 0; d < nd; d++) if (s->B[d].m > most) most = s->B[d].m;
   if (top >= minlevel) {
     EACH (bmg_blocks_bottom (dim, g, Delta, minlevel, top, B, s->dims, s->periodic, nrelax, top < L,
                              s->stream[d]));
@@ -575,6 +578,20 @@ static int shard_cycle (bmg_shard * s, blk_t * k, int nrelax, int minlevel, int 
   }
   const bmg_geom none = {0};
   for (int l = top + 1; l <= maxlevel; l++) {
+    if (dim == 2 && !jacobi && l >= 1 && nrelax >= 1 && cells_of (dim, l)*most <= BMG_BLOCKS_TILE_CELLS) {
+      int in = l == minlevel ? BMG_BLOCKS_ZERO : odd ? BMG_BLOCKS_COARSE_DA2 : BMG_BLOCKS_COARSE_DA;
+      int out = BMG_BLOCKS_DA;
+      for (int i = 0; i < nrelax; i += BMG_BLOCKS_SWEEPS) {
+        const int left = nrelax - i, ns = left < BMG_BLOCKS_SWEEPS ? left : BMG_BLOCKS_SWEEPS;
+        EACH (bmg_blocks_tile (l == minlevel ? none : g[l - 1], g[l], l, B, s->dims, s->periodic,
+                               Delta[l], in, out, ns, ns == left, s->stream[d]));
+        *launches += nd;
+        in = out;
+        out = out == BMG_BLOCKS_DA ? BMG_BLOCKS_DA2 : BMG_BLOCKS_DA;
+      }
+      odd = in == BMG_BLOCKS_DA2;
+      continue;
+    }
     EACH (bmg_blocks_prolong (dim, odd, l == minlevel ? none : g[l - 1], g[l], l, B, s->stream[d]));
     *launches += nd;
     odd = 0;

@@ -173,7 +173,7 @@ def test_blocks_of_one_cell():
 
 @pytest.mark.parametrize("relax", ["rbgs", "jacobi"])
 @pytest.mark.parametrize("dim,depth,dims", [(1, 4, (3,)), (2, 4, (3, 1)), (2, 5, (3, 1)), (2, 3, (5, 3)),
-                                            (3, 3, (3, 1, 1))])
+                                            (2, 6, (3, 1)), (2, 5, (5, 3)), (3, 3, (3, 1, 1))])
 def test_repeated_blocks_equal_one_block(dim, depth, dims, relax):
     """A periodic domain of equal blocks, their number not a power of two:
     every block is the periodic solve of one block (the coarse levels of all
@@ -200,3 +200,35 @@ def test_repeated_blocks_equal_one_block(dim, depth, dims, relax):
     for key in ("i", "nrelax", "resb", "resa"):
         assert sn[key] == s1[key], (key, sn, s1)
     np.testing.assert_array_equal(an, np.tile(a1, dims))
+
+
+def test_tiles_and_passes_bit_identical():
+    """Levels on either side of the size up to which tiles take several
+    sweeps per launch."""
+    import helpers
+    prob = helpers.random_problem(2, 10, np.random.default_rng(10), lam="field",
+                                  bc={0: ("dirichlet", 0.5), 1: ("neumann", -0.25),
+                                      2: ("dirichlet", -1.0), 3: ("neumann", 0.75)})
+    compare(prob, (2, 2), "rbgs", 1e-2*np.abs(prob["b"]).max())
+
+
+def test_coarsest_level_of_tiles():
+    """minlevel above the single-CTA levels: the cycle starts from zero on a
+    level of tiles.  -laplacian + |lambda| is an M-matrix, whose inverse's
+    maximum norm is at most 1/|lambda|: two solutions differ by at most the
+    sum of their residuals over |lambda|."""
+    sols = []
+    lam = 1e4
+    b = np.random.default_rng(3).standard_normal((256, 256))
+    for minlevel in (7, 1):
+        sg = ShardedGrid(2, 7, dims=(2, 2), relax="rbgs")
+        a = sg.scalar()
+        for side in ("right", "left", "top", "bottom"):
+            a.bc(side, "dirichlet", 0.0)
+        a.set(np.zeros(b.shape))
+        st = sg.poisson(a, sg.scalar(b), lambda_=sg.const_scalar(-lam), tolerance=1e-7, minlevel=minlevel)
+        assert st["status"] == 0 and st["resa"] <= 1e-7, st
+        sols.append((a.get(), st["resa"]))
+        sg.close()
+    (a7, r7), (a1, r1) = sols
+    assert np.abs(a7 - a1).max() <= (r7 + r1)/lam*(1. + 1e-6)
