@@ -358,7 +358,9 @@ __global__ void __launch_bounds__ (VB_THREADS, 1) k_visc_bottom (const __grid_co
     bool own[2];
     int ci[2], cj[2], ck[2];
     VCell<DIM> cf[2];
-    double rd[2][DIM], den[2][DIM];
+    double rd[2][DIM], den[2][DIM], y[2][DIM];
+    int goff[2][DIM], gside[2][DIM];    /* the cell's image per direction: offset (0: none), side */
+    bool plain = false;                 /* a divisor outside exact_quotient's range */
 #pragma unroll
     for (int o = 0; o < 2; o++) {
       own[o] = tid < (n > 1 ? half : o == 0 ? 1 : 0);
@@ -375,19 +377,59 @@ __global__ void __launch_bounds__ (VB_THREADS, 1) k_visc_bottom (const __grid_co
         for (int c = 0; c < DIM; c++) {
           rd[o][c] = P.res[m].p[c][id]*(Delta*Delta);
           den[o][c] = (Delta*Delta)*1. + cf[o].s*visc_den<DIM> (c, cf[o]);
+          y[o][c] = 1./den[o][c];
+          plain = plain || divisor_unsafe (den[o][c]);
         }
       }
+      const int x[3] = {ci[o], cj[o], ck[o]};
+#pragma unroll
+      for (int e = 0; e < DIM; e++) {
+        const int st = (int) cstride<DIM> (gs, e);
+        const bool lo = x[e] == 0, hi = x[e] == n - 1;
+        gside[o][e] = 2*e + (lo ? 1 : 0);
+        goff[o][e] = !lo && !hi ? 0 : P.bc.c[0].periodic[e] ? (lo ? n : -n)*st : lo ? -st : st;
+      }
     }
+    /* value v of component c into cell id of colour t, and its images: all
+       products of the directions' (ghosts_homog's; a single cell has two
+       images per direction) */
+    auto put = [&] (int t, int c, int id, double v) {
+      U[c][id] = v;
+      if (n == 1) { ghosts_homog<DIM, double> (U[c], gs, ci[t], cj[t], ck[t], v, P.bc.c[c]); return; }
+      const int a = goff[t][0], b = goff[t][1], d = DIM == 3 ? goff[t][DIM - 1] : 0;
+      if (!(a | b | d)) return;
+      const BCH & h = P.bc.c[c];
+      const double fa = h.periodic[0] ? 1. : h.fac[gside[t][0]], fb = h.periodic[1] ? 1. : h.fac[gside[t][1]];
+      if (a) U[c][id + a] = v*fa;
+      if (b) U[c][id + b] = v*fb;
+      if (a && b) U[c][id + a + b] = v*fa*fb;
+      if (DIM == 3 && d) {
+        const double fd = h.periodic[2] ? 1. : h.fac[gside[t][DIM - 1]];
+        U[c][id + d] = v*fd;
+        if (a) U[c][id + a + d] = v*fa*fd;
+        if (b) U[c][id + b + d] = v*fb*fd;
+        if (a && b) U[c][id + a + b + d] = v*fa*fb*fd;
+      }
+    };
     __syncthreads ();
     for (int sw = 0; sw < P.nrelax; sw++) {
       double w[2][DIM];
 #pragma unroll
       for (int o = 0; o < 2; o++) {
         const int id = (int) cidx<DIM> (gs, ci[o], cj[o], ck[o]);
-        if (own[o])
+        if (own[o]) {
+          double nn[DIM];
+          bool unsafe = plain;
 #pragma unroll
-          for (int c = 0; c < DIM; c++)
-            w[o][c] = (cf[o].s*visc_A<DIM> (gs, c, id, U, cf[o]) + rd[o][c])/den[o][c];
+          for (int c = 0; c < DIM; c++) {
+            nn[c] = cf[o].s*visc_A<DIM> (gs, c, id, U, cf[o]) + rd[o][c];
+            w[o][c] = exact_quotient (nn[c], den[o][c], y[o][c]);
+            unsafe = unsafe || quotient_unsafe (nn[c]);
+          }
+          if (__any_sync (__activemask (), unsafe))
+#pragma unroll
+            for (int c = 0; c < DIM; c++) w[o][c] = nn[c]/den[o][c];
+        }
         /* a Jacobi sweep computes both cells before it stores either */
         if (P.jacobi && o == 0) continue;
         __syncthreads ();
@@ -397,9 +439,7 @@ __global__ void __launch_bounds__ (VB_THREADS, 1) k_visc_bottom (const __grid_co
           const int it = (int) cidx<DIM> (gs, ci[t], cj[t], ck[t]);
 #pragma unroll
           for (int c = 0; c < DIM; c++) {
-            const double v = P.jacobi ? (U[c][it] + 2.*w[t][c])/3. : w[t][c];
-            U[c][it] = v;
-            ghosts_homog<DIM, double> (U[c], gs, ci[t], cj[t], ck[t], v, P.bc.c[c]);
+            put (t, c, it, P.jacobi ? (U[c][it] + 2.*w[t][c])/3. : w[t][c]);
           }
         }
         __syncthreads ();
