@@ -94,36 +94,6 @@ __device__ __forceinline__ double visc_w (const bmg_geom & g, int c, long long i
   return (q.s*A + R*(Delta*Delta))/((Delta*Delta)*1. + q.s*visc_den<DIM> (c, q));
 }
 
-/* ghosts_homog without its tables, which live in local memory: a cell of a
-   level of n > 1 has at most one image per direction */
-template <int DIM>
-__device__ __forceinline__ void visc_ghosts (double * f, const bmg_geom & g, int i, int j, int k, double v,
-                                             const BCH & bc)
-{
-  const int n = g.n;
-  if (!on_boundary<DIM> (n, i, j, k)) return;
-  if (n == 1) { ghosts_homog<DIM, double> (f, g, i, j, k, v, bc); return; }
-  const int x[3] = {i, j, k};
-  long long off[3];
-  double fac[3];
-#pragma unroll
-  for (int e = 0; e < 3; e++) {
-    off[e] = 0; fac[e] = 1.;
-    if (e < DIM && (x[e] == 0 || x[e] == n - 1)) {
-      const long long st = cstride<DIM> (g, e);
-      off[e] = bc.periodic[e] ? (x[e] == 0 ? n : -n)*st : x[e] == 0 ? -st : st;
-      if (!bc.periodic[e]) fac[e] = x[e] == 0 ? bc.fac[2*e + 1] : bc.fac[2*e];
-    }
-  }
-  double * c = f + cidx<DIM> (g, i, j, k);
-#pragma unroll
-  for (int m = 1; m < 1 << DIM; m++) {
-    const bool a = m & 1, b = m & 2, d = m & 4;
-    if ((a && !off[0]) || (b && !off[1]) || (d && !off[2])) continue;
-    c[(a ? off[0] : 0) + (b ? off[1] : 0) + (d ? off[2] : 0)] = v*(a ? fac[0] : 1.)*(b ? fac[1] : 1.)*(d ? fac[2] : 1.);
-  }
-}
-
 /* One pass of relax_viscosity over a level, from IN into OUT (the next pass
    goes back): colour 0 / 1 updates the red / black cells of every component
    from the values before the pass (the stencil reads diagonal neighbours of
@@ -186,9 +156,9 @@ __global__ void k_visc_pass (bmg_geom g, int colour, VecP IN, VecP OUT, VecP R, 
     double * f = OUT.p[c];
     if (2*q + 1 < n) *(double2 *) (f + id0) = make_double2 (v[0][c], v[1][c]);
     else f[id0] = v[0][c];
-    visc_ghosts<DIM> (f, g, i, j, k, v[0][c], bc.c[c]);
+    ghosts_homog<DIM, double> (f, g, i, j, k, v[0][c], bc.c[c]);
     if (2*q + 1 < n)
-      visc_ghosts<DIM> (f, g, i, DIM == 2 ? j + 1 : j, DIM == 3 ? k + 1 : k, v[1][c], bc.c[c]);
+      ghosts_homog<DIM, double> (f, g, i, DIM == 2 ? j + 1 : j, DIM == 3 ? k + 1 : k, v[1][c], bc.c[c]);
   }
 }
 
@@ -250,7 +220,7 @@ __global__ void k_visc_prolong (bmg_geom gc, bmg_geom gf, VecP C, VecP F, VecB b
   for (int c = 0; c < DIM; c++) {
     const double v = visc_bilinear<DIM> (gc, C.p[c], i, j, k);
     F.p[c][cidx<DIM> (gf, i, j, k)] = v;
-    visc_ghosts<DIM> (F.p[c], gf, i, j, k, v, bc.c[c]);
+    ghosts_homog<DIM, double> (F.p[c], gf, i, j, k, v, bc.c[c]);
   }
 }
 
