@@ -122,7 +122,7 @@ __global__ void k_relax3_pair (bmg_geom g, T * out, const T * in, const T * __re
   const T v = nn/d;
   out[id] = v;
   /* the shorter code where FP64 levels are bound by HBM (256^3: 33.7 -> 32.1
-     us per pass), the quicker one in FP32 (64^3 mixed solve 1.02 -> 0.99 ms) */
+     us per pass) */
   if (sizeof (T) == 8) ghosts_homog_any<3, T> (out, g, i, j, 2*q + o, v, bc);
   else ghosts_homog<3, T> (out, g, i, j, 2*q + o, v, bc);
   if (COR) {
