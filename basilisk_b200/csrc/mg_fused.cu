@@ -42,6 +42,7 @@
 #include <string.h>
 #include <type_traits>
 #include "mg_device.cuh"
+#include "mg_tile_box.cuh"
 
 using namespace bmgd;
 
@@ -69,6 +70,12 @@ __device__ __forceinline__ int real_face (int f, int n, int periodic)
   if (!periodic) return -1;
   int r = f % n;
   return r < 0 ? r + n : r;
+}
+
+/* whether the W x W region at (i0, j0) reaches beyond a side of the box */
+__device__ __forceinline__ bool beyond_box (int i0, int j0, int W, int n, int px, int py)
+{
+  return (!px && (i0 < 0 || i0 + W > n)) || (!py && (j0 < 0 || j0 + W > n));
 }
 
 /* Shared-memory tile of TS x TS cells plus a 2S halo, stored split by
@@ -248,33 +255,6 @@ __device__ __forceinline__ void own_ghosts (T * other, int p, int m0, int o, uns
     if (glo_j >= 0 && lo == 2*e && (v >> e & 1u)) other[p*M + (glo_j >> 1)] = nv[e]*T(bc.fac[3]);
     if (ghi_j < W && hi == 2*e && (v >> e & 1u)) other[p*M + (ghi_j >> 1)] = nv[e]*T(bc.fac[2]);
   }
-}
-
-/* the same for a thread whose K cells of each colour are columns q0 .. q0 +
-   2K - 1 of row p, m0 = q0/2, of a level whose sides are multiples of 2K: the
-   sides are known for the launch (0 for most threads) */
-template <int K>
-__device__ __forceinline__ unsigned box_sides (int gi, int gj, int p, int q0, int W, int n, int px, int py,
-                                               bool ok)
-{
-  if (!ok) return 0;
-  return (!px && gi == 0 && p > 0 ? 1u : 0u) | (!px && gi == n - 1 && p + 1 < W ? 2u : 0u) |
-    (!py && gj == 0 && q0 > 0 ? 4u : 0u) | (!py && gj + 2*K == n && q0 + 2*K < W ? 8u : 0u);
-}
-
-template <int M, typename T, int K>
-__device__ __forceinline__ void side_ghosts (T * other, unsigned sides, int p, int m0, int o,
-                                             const T (& nv)[K], const BCH & bc)
-{
-  if (!sides) return;
-  T * c = other + p*M + m0;
-#pragma unroll
-  for (int e = 0; e < K; e++) {
-    if (sides & 1u) c[e - M] = nv[e]*T(bc.fac[1]);
-    if (sides & 2u) c[e + M] = nv[e]*T(bc.fac[0]);
-  }
-  if ((sides & 4u) && o == 0) c[-1] = nv[0]*T(bc.fac[3]);
-  if ((sides & 8u) && o == 1) c[K] = nv[K - 1]*T(bc.fac[2]);
 }
 
 /* the ghost images of the cells (i, j) .. (i, j + 3) of a level of n > 4
@@ -679,10 +659,14 @@ k_relax_tile2d_w (bmg_geom g, float * __restrict__ out, const float * __restrict
     /* outside the domain */
 #pragma unroll
     for (int q = 0; q < 8; q++) r8[q] = xl8[q] = xu8[q] = yl8[q] = yl8[q + 1] = l8[q] = 0.f;
+  const int cq = (base + p) & 1;                /* colour of the even columns */
+  if (beyond_box (i0, j0, W, n, px, py)) {
+    zero_outside<M, float, 4> (sa + cq*WM, sa + (cq ^ 1)*WM, ok, p, m0);
+    __syncthreads ();
+  }
   /* the iterate is the previous launch's output: its loads are issued
      before the weights are computed, so that both round trips overlap */
   grid_dependency_wait ();
-  const int cq = (base + p) & 1;                /* colour of the even columns */
   {
     float v8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (ok) {
@@ -697,10 +681,7 @@ k_relax_tile2d_w (bmg_geom g, float * __restrict__ out, const float * __restrict
       }
     }
     const float ev[4] = {v8[0], v8[2], v8[4], v8[6]}, od[4] = {v8[1], v8[3], v8[5], v8[7]};
-    *(float4 *) (sa + cq*WM + p*M + m0) = make_float4 (ev[0], ev[1], ev[2], ev[3]);
-    *(float4 *) (sa + (cq ^ 1)*WM + p*M + m0) = make_float4 (od[0], od[1], od[2], od[3]);
-    side_ghosts<M> (sa + (cq ^ 1)*WM, sides, p, m0, 0, ev, bc);
-    side_ghosts<M> (sa + cq*WM, sides, p, m0, 1, od, bc);
+    stage_cells<M> (sa + cq*WM, sa + (cq ^ 1)*WM, ok, sides, p, m0, ev, od, bc);
   }
   /* weights of cell e of colour c: column 2e + o_c of the eight */
   float wxl[2][4], wxu[2][4], wyl[2][4], wyr[2][4], be[2][4];
@@ -729,16 +710,17 @@ k_relax_tile2d_w (bmg_geom g, float * __restrict__ out, const float * __restrict
   /* the colour passes.  Rows shrink by one per pass (whole warps drop out);
      columns do not: a cell next to the staged region's edge may be updated
      from stale neighbours, but staleness moves inward by one cell per pass
-     and never reaches the TS x TS interior after 2S passes, so only cells
-     outside the domain are masked.  Shared memory is addressed by 32-bit byte offsets with the
-     row offsets as immediates. */
+     and never reaches the TS x TS interior after 2S passes; threads outside
+     the box take no part.  Shared memory is addressed by 32-bit byte offsets
+     with the row offsets as immediates. */
   const unsigned sbase = (unsigned) __cvta_generic_to_shared (sa);
   const int o0 = (base ^ p) & 1;               /* column offset of colour 0 in row p */
+  const int passes = ok ? min (p, W - 1 - p) : 0;
   for (int sw = 0; sw < nsweeps; sw++)
 #pragma unroll
     for (int c = 0; c < 2; c++) {
       const int k = 2*sw + c;
-      if (p >= k + 1 && p < W - k - 1) {
+      if (k < passes) {
         const int o = o0 ^ c;
         /* the other colour's quad at rows p - 1, p, p + 1 and its left or
            right neighbour in row p */
@@ -754,7 +736,7 @@ k_relax_tile2d_w (bmg_geom g, float * __restrict__ out, const float * __restrict
           nv[e] = fmaf (wyr[c][e], v[e + 1], fmaf (wyl[c][e], v[e],
                   fmaf (wxu[c][e], dnv[e], fmaf (wxl[c][e], upv[e], be[c][e]))));
         const unsigned aw = sbase + 4u*(c*WM + p*M + m0);
-        if (ok) sts_f4 (aw, make_float4 (nv[0], nv[1], nv[2], nv[3]));
+        sts_f4 (aw, make_float4 (nv[0], nv[1], nv[2], nv[3]));
         side_ghosts<M> (sa + (c ^ 1)*WM, sides, p, m0, o, nv, bc);
       }
       __syncthreads ();
@@ -1231,16 +1213,20 @@ k_relax_tile2d_x4 (bmg_geom g, double * __restrict__ out, const double * __restr
     }
   }
   else
-    /* outside the domain (never stored): a quotient of ordinary numbers,
-       the division of zeros being several times slower */
+    /* outside the box, where no pass stores: a reciprocal of an ordinary
+       number (that of zero is several times slower) */
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       r4[q] = -1./D2;
       xl4[q] = l4[q] = yl4[q] = yl4[q + 1] = 0.;
       xu4[q] = 1.;
     }
-  grid_dependency_wait ();
   const int cq = (base + p) & 1;
+  if (beyond_box (i0, j0, W, n, px, py)) {
+    zero_outside<M, double, 2> (sa + cq*WM, sa + (cq ^ 1)*WM, ok, p, m0);
+    __syncthreads ();
+  }
+  grid_dependency_wait ();
   {
     double v4[4] = {0., 0., 0., 0.};
     if (ok) {
@@ -1252,11 +1238,8 @@ k_relax_tile2d_x4 (bmg_geom g, double * __restrict__ out, const double * __restr
         v4[0] = va.x; v4[1] = va.y; v4[2] = va.z; v4[3] = va.w;
       }
     }
-    const Quad<double> va = {v4[0], v4[1], v4[2], v4[3]};
-    put_quad (sa + cq*WM, sa + (cq ^ 1)*WM, p*M + m0, va);
     const double ev[2] = {v4[0], v4[2]}, od[2] = {v4[1], v4[3]};
-    side_ghosts<M> (sa + (cq ^ 1)*WM, sides, p, m0, 0, ev, bc);
-    side_ghosts<M> (sa + cq*WM, sides, p, m0, 1, od, bc);
+    stage_cells<M> (sa + cq*WM, sa + (cq ^ 1)*WM, ok, sides, p, m0, ev, od, bc);
   }
   /* -Delta^2 b and -Delta^2 lambda in place of b and lambda, and the
      reciprocals of the diagonals */
@@ -1311,11 +1294,12 @@ k_relax_tile2d_x4 (bmg_geom g, double * __restrict__ out, const double * __restr
     if (__any_sync (__activemask (), plain))
 #pragma unroll
       for (int e = 0; e < 2; e++) nv[e] = nn[e]/diag (e);
-    if (ok) sts_d2 (aw, make_double2 (nv[0], nv[1]));
+    sts_d2 (aw, make_double2 (nv[0], nv[1]));
     side_ghosts<M> (sa + (c ^ 1)*WM, sides, p, m0, O, nv, bc);
   };
+  const int passes = ok ? min (p, W - 1 - p) : 0;
   for (int k = 0; k < 2*nsweeps; k++) {
-    if (p >= k + 1 && p < W - k - 1) {
+    if (k < passes) {
       if ((o0 ^ k) & 1) update (std::integral_constant<int, 1> (), k & 1);
       else update (std::integral_constant<int, 0> (), k & 1);
     }
@@ -1397,8 +1381,12 @@ k_relax_tile2d_c (bmg_geom g, double * __restrict__ out, const double * __restri
       cnb[1][e] = swap ? v0 : v1;
     }
   }
-  grid_dependency_wait ();
   const int cq = (base + p) & 1;
+  if (beyond_box (i0, j0, W, n, px, py)) {
+    zero_outside<M, double, 4> (sa + cq*WM, sa + (cq ^ 1)*WM, ok, p, m0);
+    __syncthreads ();
+  }
+  grid_dependency_wait ();
   {
     double v8[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
     if (ok) {
@@ -1410,12 +1398,8 @@ k_relax_tile2d_c (bmg_geom g, double * __restrict__ out, const double * __restri
         v8[4] = vb.x; v8[5] = vb.y; v8[6] = vb.z; v8[7] = vb.w;
       }
     }
-    double * se = sa + cq*WM + p*M + m0, * so = sa + (cq ^ 1)*WM + p*M + m0;
-    *(double2 *) se = make_double2 (v8[0], v8[2]); *(double2 *) (se + 2) = make_double2 (v8[4], v8[6]);
-    *(double2 *) so = make_double2 (v8[1], v8[3]); *(double2 *) (so + 2) = make_double2 (v8[5], v8[7]);
     const double ev[4] = {v8[0], v8[2], v8[4], v8[6]}, od[4] = {v8[1], v8[3], v8[5], v8[7]};
-    side_ghosts<M> (sa + (cq ^ 1)*WM, sides, p, m0, 0, ev, bc);
-    side_ghosts<M> (sa + cq*WM, sides, p, m0, 1, od, bc);
+    stage_cells<M> (sa + cq*WM, sa + (cq ^ 1)*WM, ok, sides, p, m0, ev, od, bc);
   }
   double d = (-lamc)*D2;
   d += axc + axc;
@@ -1426,11 +1410,12 @@ k_relax_tile2d_c (bmg_geom g, double * __restrict__ out, const double * __restri
 
   const unsigned sbase = (unsigned) __cvta_generic_to_shared (sa);
   const int o0 = (base ^ p) & 1;
+  const int passes = ok ? min (p, W - 1 - p) : 0;
   for (int sw = 0; sw < nsweeps; sw++)
 #pragma unroll
     for (int c = 0; c < 2; c++) {
       const int k = 2*sw + c;
-      if (p >= k + 1 && p < W - k - 1) {
+      if (k < passes) {
         const int o = o0 ^ c;
         const unsigned aup = sbase + 8u*((c ^ 1)*WM + (p - 1)*M + m0);
         const double2 u0 = lds_d2<0> (aup), u1 = lds_d2<16> (aup);
@@ -1454,10 +1439,8 @@ k_relax_tile2d_c (bmg_geom g, double * __restrict__ out, const double * __restri
 #pragma unroll
           for (int e = 0; e < 4; e++) nv[e] = nn[e]/d;
         const unsigned aw = sbase + 8u*(c*WM + p*M + m0);
-        if (ok) {
-          sts_d2 (aw, make_double2 (nv[0], nv[1]));
-          sts_d2 (aw + 16, make_double2 (nv[2], nv[3]));
-        }
+        sts_d2 (aw, make_double2 (nv[0], nv[1]));
+        sts_d2 (aw + 16, make_double2 (nv[2], nv[3]));
         side_ghosts<M> (sa + (c ^ 1)*WM, sides, p, m0, o, nv, bc);
       }
       __syncthreads ();

@@ -62,3 +62,25 @@ def test_mixed_commutes_with_half_a_period(depth, lam):
         g.close()
     assert out[0][0] == out[1][0]
     np.testing.assert_array_equal(roll(out[0][1]), out[1][1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("depth", [9, 10])
+@pytest.mark.parametrize("alpha", ["stored", "unit"])
+def test_a_solve_repeats_itself(depth, precision, alpha):
+    """The same walls, coefficients and right-hand side many times on one grid:
+    the same bits each time."""
+    p = problem(depth, "walls", None, 3)
+    if alpha == "unit":
+        p = dict(p, alpha=None)
+    g, a, b, al, lam = helpers.gpu_grid(p, relax="rbgs", precision=precision)
+    zero = np.zeros((1 << depth, 1 << depth))
+    first = None
+    for _ in range(12):
+        a.set(zero)
+        st = g.poisson(a, b, alpha=al, lambda_=lam, tolerance=1e300, nrelax=6)
+        if first is None:
+            first = (st["resa"], a.get())
+        assert st["resa"] == first[0]
+        np.testing.assert_array_equal(a.get(), first[1])
+    g.close()
