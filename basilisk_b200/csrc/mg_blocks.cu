@@ -725,7 +725,8 @@ extern "C" {
 int bmg_blocks_relax (int dim, int mode, int odd, bmg_geom g, int l, bmg_blocks B, double Delta,
                       cudaStream_t s)
 {
-  if (l < 1) return (int) cudaErrorInvalidValue;
+  /* (single cells have no colours: their images would be read in the pass) */
+  if (l < (mode == BMG_SWEEP_JACOBI ? 0 : 1)) return (int) cudaErrorInvalidValue;
   return status_of (dim == 1 ? relax_dim<1> (mode, odd, g, l, B, Delta, s)
                     : dim == 2 ? relax_dim<2> (mode, odd, g, l, B, Delta, s)
                     : relax_dim<3> (mode, odd, g, l, B, Delta, s));

@@ -171,6 +171,33 @@ def test_blocks_of_one_cell():
     sg.close()
 
 
+@pytest.mark.parametrize("dim,dims,periodic", [(1, (4,), False), (2, (2, 2), False), (2, (4, 4), True),
+                                               (3, (2, 2, 2), False)])
+def test_jacobi_on_blocks_of_one_cell_bit_identical(dim, dims, periodic):
+    """Blocks of depth 0 against the one level of a grid of dims cells."""
+    import helpers
+    k = int(math.log2(dims[0]))
+    rng = np.random.default_rng(70 + dim)
+    bc = {s: ("dirichlet", 0.5) if s % 3 else ("neumann", -0.25) for s in range(2 * dim)}
+    prob = helpers.random_problem(dim, k, rng, periodic=tuple(range(dim)) if periodic else (),
+                                  bc=None if periodic else bc, lam="field")
+    if periodic:
+        for d, c in enumerate(prob["alpha"]):    # face n of a periodic direction is face 0
+            c[(slice(None),) * d + (-1,)] = c[(slice(None),) * d + (0,)]
+    g, a, b, alpha, lam = helpers.gpu_grid(prob, relax="jacobi")
+    st = g.poisson(a, b, alpha=alpha, lambda_=lam, tolerance=1e-9, minlevel=k)
+    ref = a.get()
+    g.close()
+    sg, sa, sb, salpha, slam = sharded(prob, dims, "jacobi")
+    ss = sg.poisson(sa, sb, alpha=salpha, lambda_=slam, tolerance=1e-9)
+    got = sa.get()
+    sg.close()
+    assert ss["minlevel"] == 0
+    for key in ("status", "i", "nrelax", "resb", "resa"):
+        assert ss[key] == st[key], (key, ss, st)
+    np.testing.assert_array_equal(got, ref)
+
+
 @pytest.mark.parametrize("relax", ["rbgs", "jacobi"])
 @pytest.mark.parametrize("dim,depth,dims", [(1, 4, (3,)), (2, 4, (3, 1)), (2, 5, (3, 1)), (2, 3, (5, 3)),
                                             (2, 6, (3, 1)), (2, 5, (5, 3)), (3, 3, (3, 1, 1))])
