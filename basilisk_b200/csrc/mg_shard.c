@@ -66,7 +66,6 @@ struct bmg_shard {
   long long nhalo;            /* exchange launches */
   /* the tables of the blocks' kernels (mg_blocks.h): the host's copy, and
      each device's, written when a solve's differ from the last one's */
-  size_t tbytes;
   bmg_blk * tblk;
   bmg_blk_level * tlv;
   void * dtab[16];
@@ -385,14 +384,14 @@ static int upload_tables (bmg_shard * s, const blk_t * k)
   const size_t nlv = (size_t) (L + 1)*nb;
   const size_t olv = nb*sizeof (bmg_blk), omine = olv + nlv*sizeof (bmg_blk_level);
   const size_t bytes = omine + nb*sizeof (int);
-  if (!s->tblk) {
-    if (!(s->tblk = calloc (2, bytes))) return FAIL (BMG_ENOMEM);
-    s->tbytes = bytes;
-    for (int d = 0; d < s->ndev; d++) {
+  if (!s->tblk && !(s->tblk = calloc (2, bytes))) return FAIL (BMG_ENOMEM);
+  /* (each on its own: an allocation that failed in one solve is tried again
+     in the next) */
+  for (int d = 0; d < s->ndev; d++)
+    if (!s->dtab[d]) {
       CKS (cudaSetDevice (s->dev[d]));
       CKS (cudaMalloc (&s->dtab[d], bytes));
     }
-  }
   /* the second half of the host buffer takes this solve's tables */
   char * cur = (char *) s->tblk, * now = cur + bytes;
   memset (now, 0, bytes);
