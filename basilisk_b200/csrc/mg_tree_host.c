@@ -438,8 +438,10 @@ static int dep_visit (depset * s, int m, int i, int j)
    by level, colour and kind (so that every level's relaxation set, its own
    cells and the leaves below, is even too), and per level the records of its
    lists by owning rank.  list, rules: the stages' cells and ghosts.  Leaves
-   tc.slots = 0 when the closure has more stages than a record holds. */
-static int cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h, const uint32_t * list,
+   tc.slots = 0, for the interpreter to run the cycle, when the closure has
+   more stages than a record holds and when there is no memory for the
+   records. */
+static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h, const uint32_t * list,
                           const bmg_tree_rule * rules)
 {
   const int D = t->depth, NR = BMG_TC_RANKS;
@@ -447,7 +449,7 @@ static int cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h,
   for (int k = 0; k < 4; k++) { cudaFree (t->dtc[k]); t->dtc[k] = NULL; }
   long total = 0;
   for (int l = 0; l <= D; l++) {
-    if (t->dep[l].n > BMG_TC_STAGES) return BMG_OK;
+    if (t->dep[l].n > BMG_TC_STAGES) return;
     total += t->act[l].n + t->rl[l].n;
     for (long k = 0; k < t->dep[l].n; k++) {
       const tdep * d = &t->deps[t->dep[l].off + k];
@@ -580,10 +582,13 @@ static int cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h,
     if (cudaMalloc (&t->dtc[k], sz[k] + 16) != cudaSuccess ||
         cudaMemcpy (t->dtc[k], hp[k], sz[k], cudaMemcpyHostToDevice) != cudaSuccess) err = 1;
   t->tc.lv = t->dtc[0]; t->tc.own = t->dtc[1]; t->tc.id = t->dtc[2]; t->tc.src = t->dtc[3];
-  if (err) { cudaGetLastError (); t->tc.slots = 0; }
+  if (err) {
+    cudaGetLastError ();
+    for (int k = 0; k < 4; k++) { cudaFree (t->dtc[k]); t->dtc[k] = NULL; }
+    memset (&t->tc, 0, sizeof t->tc);
+  }
   for (int l = 0; l <= D; l++) free (slot[l]);
   free (lv); free (own); free (id); free (src);
-  return err == 1 ? BMG_ENOMEM : BMG_OK;
 }
 
 /* the stages of every level, uploaded; h: the host cell lists */
@@ -671,9 +676,9 @@ static int depend (bmg_grid * g, struct bmg_tree * t, const uint32_t * h)
        (nrules && cudaMemcpy (t->ddrules, rules, nrules*sizeof (bmg_tree_rule), cudaMemcpyHostToDevice)
         != cudaSuccess)))
     s.err = 1;
-  int r = s.err ? BMG_ENOMEM : cycle_records (g, t, h, list, rules);
+  if (!s.err) cycle_records (g, t, h, list, rules);
   free (list); free (rules);
-  return r;
+  return s.err ? BMG_ENOMEM : BMG_OK;
 }
 
 /* flags of halo cells and prolongation leaves, cell lists, ghost rules:
