@@ -153,6 +153,8 @@ int bmg_tree_launch_interp_mixed (const bmg_tree_op * ops, int nops, const bmg_t
    the level of a relaxed cell, the kind of a stage's cell. */
 #define BMG_TC_RANKS 16
 #define BMG_TC_STAGES 6
+/* most slots of a rank: FP32 values in the shared memory of a CTA */
+#define BMG_TC_SLOTS (227*1024/4)
 enum { BMG_TC_PROLONG = 0, BMG_TC_RED, BMG_TC_BLACK, BMG_TC_CELLS };
 enum { BMG_TC_RESTRICT = 0, BMG_TC_HALO, BMG_TC_GHOST };
 typedef struct {

@@ -382,16 +382,29 @@ typedef struct {
   struct bmg_tree * t;
   int l, err;
   unsigned char * mark[TMAX + 1];    /* 0: not visited, else stage + 1 */
-  uint32_t * cell;                   /* the visited cells, and their stages */
+  uint32_t * cell;                   /* the visited cells */
   long n, cap;
 } depset;
 
-static int dep_inset (const depset * s, int m, int i, int j)
+static inline int dep_inset (const depset * s, int m, int i, int j)
 {
   const int n = 1 << m;
   if (i < 0 || j < 0 || i >= n || j >= n) return 0;
   const unsigned char f = s->t->fl[m][HX (m, i, j)];
   return (f & BMG_T_ACTIVE) && (m == s->l || (f & BMG_T_LEAF));
+}
+
+static int dep_mark (depset * s, unsigned char * mk, int m, int i, int j, int d)
+{
+  *mk = (unsigned char) (d + 1);
+  if (s->n == s->cap) {
+    const long cap = 2*s->cap + 1024;
+    uint32_t * c = realloc (s->cell, cap*sizeof (uint32_t));
+    if (!c) { s->err = 1; return d; }
+    s->cell = c; s->cap = cap;
+  }
+  s->cell[s->n++] = pack (m, i, j);
+  return d;
 }
 
 /* the stage of a cell: 0 in the set (or never computed), else after its
@@ -406,7 +419,7 @@ static int dep_visit (depset * s, int m, int i, int j)
 #define SRC(m_, i_, j_) do { const int q_ = dep_visit (s, m_, i_, j_); if (q_ > d) d = q_; } while (0)
   if (i < 0 || j < 0 || i >= n || j >= n) {
     bmg_tree_rule r;
-    if (!ghost_rule (s->t, m, i, j, &r)) { *mk = 1; return 0; }
+    if (!ghost_rule (s->t, m, i, j, &r)) return dep_mark (s, mk, m, i, j, 0);
     SRC (m, (int) ((r.inner >> 14) & 0x3FFF) - 1, (int) (r.inner & 0x3FFF) - 1);
   }
   else {
@@ -418,19 +431,10 @@ static int dep_visit (depset * s, int m, int i, int j)
       const int pi = i >> 1, pj = j >> 1, cx = (i & 1) ? 1 : -1, cy = (j & 1) ? 1 : -1;
       SRC (m - 1, pi, pj); SRC (m - 1, pi + cx, pj); SRC (m - 1, pi, pj + cy); SRC (m - 1, pi + cx, pj + cy);
     }
-    else { *mk = 1; return 0; }
+    else return dep_mark (s, mk, m, i, j, 0);
   }
 #undef SRC
-  d++;
-  *mk = (unsigned char) (d + 1);
-  if (s->n == s->cap) {
-    const long cap = 2*s->cap + 1024;
-    uint32_t * c = realloc (s->cell, cap*sizeof (uint32_t));
-    if (!c) { s->err = 1; return d; }
-    s->cell = c; s->cap = cap;
-  }
-  s->cell[s->n++] = pack (m, i, j);
-  return d;
+  return dep_mark (s, mk, m, i, j, d + 1);
 }
 
 /* The records of the cycle in distributed shared memory: a slot of one of
@@ -438,24 +442,26 @@ static int dep_visit (depset * s, int m, int i, int j)
    by level, colour and kind (so that every level's relaxation set, its own
    cells and the leaves below, is even too), and per level the records of its
    lists by owning rank.  list, rules: the stages' cells and ghosts.  Leaves
-   tc.slots = 0, for the interpreter to run the cycle, when the closure has
-   more stages than a record holds and when there is no memory for the
-   records. */
+   tc.slots = 0, for the interpreter to run the cycle, when the tree has too
+   many cells for any form's slots, when the closure has more stages than a
+   record holds, and when there is no memory for the records. */
 static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h, const uint32_t * list,
                           const bmg_tree_rule * rules)
 {
   const int D = t->depth, NR = BMG_TC_RANKS;
   memset (&t->tc, 0, sizeof t->tc);
   for (int k = 0; k < 4; k++) { cudaFree (t->dtc[k]); t->dtc[k] = NULL; }
-  long total = 0;
+  long total = 0, active = 0;
   for (int l = 0; l <= D; l++) {
     if (t->dep[l].n > BMG_TC_STAGES) return;
     total += t->act[l].n + t->rl[l].n;
+    active += t->act[l].n;
     for (long k = 0; k < t->dep[l].n; k++) {
       const tdep * d = &t->deps[t->dep[l].off + k];
       total += d->nrest + d->nhalo + d->rules.n;
     }
   }
+  if (!t->interp || active > (long) NR*BMG_TC_SLOTS) return;
   int err = 0;
   uint32_t * slot[TMAX + 1], next[BMG_TC_RANKS];
   memset (slot, 0, sizeof slot);
@@ -527,41 +533,45 @@ static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h
       const long n = kind == BMG_TC_PROLONG ? (l > 0 ? t->act[l].n : 0)
         : kind == BMG_TC_RED ? t->rl1[l] : kind == BMG_TC_BLACK ? t->rl[l].n - t->rl1[l]
         : q->nrest + q->nhalo + q->rules.n;
-      for (uint32_t r = 0; r < (uint32_t) NR; r++) {
+      /* counted, then dealt to the ranks in order */
+      long at[BMG_TC_RANKS];
+#define ENTRY(k) (k < listed ? cells[k] : rules[q->rules.off + k - listed].ghost)
+      const long listed = q ? q->nrest + q->nhalo : n;
+      for (long k = 0; k < n; k++) lv[l].n[kind][SLOT (ENTRY (k)) >> 16]++;
+      for (int r = 0; r < NR; r++) {
         lv[l].off[kind][r] = (uint32_t) w;
-        for (long k = 0; k < n; k++) {
-          const int ghost = q && k >= q->nrest + q->nhalo;
-          const bmg_tree_rule * gr = ghost ? &rules[q->rules.off + k - q->nrest - q->nhalo] : NULL;
-          const uint32_t e = ghost ? gr->ghost : cells[k], sl = SLOT (e);
-          if (sl >> 16 != r) continue;
-          const int m = LVL (e), i = CI (e), j = CJ (e);
-          uint32_t * s = src + 4*w;
-          const int halo = q && !ghost && k >= q->nrest;
-          uint32_t aux = 0;
-          if (ghost) {
-            s[0] = SLOT (gr->inner); s[1] = gr->kind_sides; s[2] = s[3] = 0;
-            aux = BMG_TC_GHOST;
-          }
-          else if (kind == BMG_TC_PROLONG || halo) {
-            const int pi = i >> 1, pj = j >> 1, cx = (i & 1) ? 1 : -1, cy = (j & 1) ? 1 : -1;
-            s[0] = CODE (m - 1, pi, pj, r); s[1] = CODE (m - 1, pi + cx, pj, r);
-            s[2] = CODE (m - 1, pi, pj + cy, r); s[3] = CODE (m - 1, pi + cx, pj + cy, r);
-            aux = BMG_TC_HALO;
-          }
-          else if (q) {
-            for (int c = 0; c < 4; c++) s[c] = CODE (m + 1, 2*i + (c >> 1), 2*j + (c & 1), r);
-            aux = BMG_TC_RESTRICT;
-          }
-          else {
-            s[0] = CODE (m, i - 1, j, r); s[1] = CODE (m, i + 1, j, r);
-            s[2] = CODE (m, i, j - 1, r); s[3] = CODE (m, i, j + 1, r);
-            id[w] = (uint32_t) (g->off64[m] + (size_t) (i + 1)*g->g64[m].P + g->g64[m].xo + j);
-            aux = (uint32_t) m;
-          }
-          own[w++] = (sl & 0xffff) | aux << 16;
-        }
-        lv[l].n[kind][r] = (uint32_t) (w - lv[l].off[kind][r]);
+        at[r] = w;
+        w += lv[l].n[kind][r];
       }
+      for (long k = 0; k < n; k++) {
+        const bmg_tree_rule * gr = k < listed ? NULL : &rules[q->rules.off + k - listed];
+        const uint32_t e = ENTRY (k), sl = SLOT (e), r = sl >> 16;
+        const int m = LVL (e), i = CI (e), j = CJ (e);
+        uint32_t * s = src + 4*at[r];
+        uint32_t aux = 0;
+        if (gr) {
+          s[0] = SLOT (gr->inner); s[1] = gr->kind_sides; s[2] = s[3] = 0;
+          aux = BMG_TC_GHOST;
+        }
+        else if (kind == BMG_TC_PROLONG || (q && k >= q->nrest)) {
+          const int pi = i >> 1, pj = j >> 1, cx = (i & 1) ? 1 : -1, cy = (j & 1) ? 1 : -1;
+          s[0] = CODE (m - 1, pi, pj, r); s[1] = CODE (m - 1, pi + cx, pj, r);
+          s[2] = CODE (m - 1, pi, pj + cy, r); s[3] = CODE (m - 1, pi + cx, pj + cy, r);
+          aux = BMG_TC_HALO;
+        }
+        else if (q) {
+          for (int c = 0; c < 4; c++) s[c] = CODE (m + 1, 2*i + (c >> 1), 2*j + (c & 1), r);
+          aux = BMG_TC_RESTRICT;
+        }
+        else {
+          s[0] = CODE (m, i - 1, j, r); s[1] = CODE (m, i + 1, j, r);
+          s[2] = CODE (m, i, j - 1, r); s[3] = CODE (m, i, j + 1, r);
+          id[at[r]] = (uint32_t) (g->off64[m] + (size_t) (i + 1)*g->g64[m].P + g->g64[m].xo + j);
+          aux = (uint32_t) m;
+        }
+        own[at[r]++] = (sl & 0xffff) | aux << 16;
+      }
+#undef ENTRY
     }
     for (int r = 0; r < NR; r++) {
       const int n = (int) (lv[l].n[BMG_TC_RED][r] + lv[l].n[BMG_TC_BLACK][r]);
@@ -591,6 +601,12 @@ static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h
   free (lv); free (own); free (id); free (src);
 }
 
+/* a cell that a pass reads (most are in the set) */
+static inline void dep_need (depset * s, int m, int i, int j)
+{
+  if (!dep_inset (s, m, i, j)) dep_visit (s, m, i, j);
+}
+
 /* the stages of every level, uploaded; h: the host cell lists */
 static int depend (bmg_grid * g, struct bmg_tree * t, const uint32_t * h)
 {
@@ -603,23 +619,22 @@ static int depend (bmg_grid * g, struct bmg_tree * t, const uint32_t * h)
   free (t->deps); t->deps = NULL;
   for (int l = 0; l <= t->depth && !s.err; l++) {
     const size_t m = (size_t) ((1 << l) + 2)*((1 << l) + 2);
-    if (!(s.mark[l] = malloc (m))) s.err = 1;
+    if (!(s.mark[l] = calloc (m, 1))) s.err = 1;
   }
   for (int l = 0; l <= t->depth && !s.err; l++) {
     s.l = l; s.n = 0;
-    for (int m = 0; m <= l; m++) memset (s.mark[m], 0, (size_t) ((1 << m) + 2)*((1 << m) + 2));
     for (long k = 0; k < t->rl[l].n; k++) {
       const uint32_t e = h[t->rl[l].off + k];
       const int m = (int) (e >> 28), i = (int) ((e >> 14) & 0x3FFF) - 1, j = (int) (e & 0x3FFF) - 1;
-      dep_visit (&s, m, i - 1, j); dep_visit (&s, m, i + 1, j);
-      dep_visit (&s, m, i, j - 1); dep_visit (&s, m, i, j + 1);
+      dep_need (&s, m, i - 1, j); dep_need (&s, m, i + 1, j);
+      dep_need (&s, m, i, j - 1); dep_need (&s, m, i, j + 1);
     }
     /* the neighbourhoods of the refined cells of level l */
     for (long k = 0; k < t->ref[l].n; k++) {
       const uint32_t e = h[t->ref[l].off + k];
       const int i = (int) ((e >> 14) & 0x3FFF) - 1, j = (int) (e & 0x3FFF) - 1;
       for (int a = -1; a <= 1; a++)
-        for (int b = -1; b <= 1; b++) dep_visit (&s, l, i + a, j + b);
+        for (int b = -1; b <= 1; b++) dep_need (&s, l, i + a, j + b);
     }
     int last = 0;
     for (long k = 0; k < s.n; k++) {
@@ -663,6 +678,11 @@ static int depend (bmg_grid * g, struct bmg_tree * t, const uint32_t * h)
           if (kind == 2) { if (ghost_rule (t, m, i, j, &rules[nrules])) { nrules++; st->rules.n++; } }
           else { list[nlist++] = e; if (kind == 0) st->nrest++; else st->nhalo++; }
         }
+    }
+    for (long k = 0; k < s.n; k++) {
+      const uint32_t e = s.cell[k];
+      const int m = (int) (e >> 28);
+      s.mark[m][HX (m, (int) ((e >> 14) & 0x3FFF) - 1, (int) (e & 0x3FFF) - 1)] = 0;
     }
   }
   for (int l = 0; l <= t->depth; l++) free (s.mark[l]);
@@ -1250,7 +1270,7 @@ static int t_iteration (bmg_grid * g, struct bmg_tree * t, const tkey * key, dou
       /* the same iteration's algorithmic bytes, from its operation list */
       opvec o = {NULL, 0, 0, 0, 0., c->ax.p != NULL, c->lam.p != NULL, 8.};
       long cyc0, cyc1;
-    r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel, &cyc0, &cyc1);
+      r_iteration (g, t, &o, key->nrelax, key->minlevel, key->maxlevel, &cyc0, &cyc1);
       victim->bytes = o.bytes;
       free (o.v);
     }
