@@ -105,6 +105,7 @@ struct bmg_tree {
   struct tgraph graphs[NTGRAPH];
   unsigned long long clock;
   int interp;                         /* run solve iterations through the interpreter */
+  int no_cycle;                       /* and their cycle too (BMG_NO_TREE_CYCLE in the environment) */
   float * ws32;                       /* mixed form: da, res, tmp, alpha x, alpha y, lambda in
                                          FP32, each an all-level array in the FP64 element layout */
 };
@@ -461,7 +462,7 @@ static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h
       total += d->nrest + d->nhalo + d->rules.n;
     }
   }
-  if (!t->interp || active > (long) NR*BMG_TC_SLOTS) return;
+  if (!t->interp || t->no_cycle || active > (long) NR*BMG_TC_SLOTS) return;
   int err = 0;
   uint32_t * slot[TMAX + 1], next[BMG_TC_RANKS];
   memset (slot, 0, sizeof slot);
@@ -874,6 +875,7 @@ int bmg_tree_refine (bmg_grid * g, bmg_refine_cond cond, void * data)
     }
     t->fl[0][HX (0, 0, 0)] = BMG_T_ACTIVE | BMG_T_LEAF;     /* init_grid (1) */
     t->interp = getenv ("BMG_NO_TREE_INTERP") == NULL && bmg_tree_interp_available ();
+    t->no_cycle = getenv ("BMG_NO_TREE_CYCLE") != NULL;
     g->tree = t;
   }
   long count = 0, pass;
