@@ -84,3 +84,22 @@ def test_a_solve_repeats_itself(depth, precision, alpha):
         assert st["resa"] == first[0]
         np.testing.assert_array_equal(a.get(), first[1])
     g.close()
+
+
+@pytest.mark.parametrize("depth", [9, 10])
+@pytest.mark.parametrize("sides", ["walls", "channel", "pipe"])
+@pytest.mark.parametrize("lam", [None, "field"])
+def test_mixed_cycle_is_the_fp64_cycle_to_rounding(depth, sides, lam):
+    """One cycle of both forms from the same start.  The sweeps contract, so
+    the forms differ by the roundings of the FP32 operations, some ten per
+    cell and pass, 2 nrelax passes on each of depth levels: at most
+    10 * 12 * 10 * 2^-24 = 7e-5 of the largest value.  A side's ghosts left
+    out of one pass change the cells along it by a quarter of their value."""
+    p = problem(depth, sides, lam, 17)
+    out = []
+    for precision in ("fp64", "mixed"):
+        g, a, b, alpha, lam_f = helpers.gpu_grid(p, relax="rbgs", precision=precision)
+        g.poisson(a, b, alpha=alpha, lambda_=lam_f, tolerance=1e300, nrelax=6, minlevel=1)
+        out.append(a.get())
+        g.close()
+    assert np.abs(out[1] - out[0]).max() <= 7e-5*np.abs(out[0]).max()
