@@ -16,13 +16,20 @@
  *                     (CTAs read halos that other CTAs own, so a launch never
  *                     writes what it reads).  The halo is recomputed
  *                     redundantly, so each array is read about once per S
- *                     sweeps instead of twice per sweep.  FP64 levels (in the
- *                     reference's evaluation order) and the small FP32
- *                     levels.
+ *                     sweeps instead of twice per sweep.  The levels of up
+ *                     to 256^2.
  *   k_relax_tile2d_w  the same temporal blocking for the large FP32 levels of
  *                     the mixed form, with each thread's cells' coefficients
  *                     divided by the diagonal once per launch and kept in
  *                     registers: only the iterate is staged.
+ *   k_relax_tile2d_x4, k_relax_tile2d_c
+ *                     the large FP64 levels, in the reference's evaluation
+ *                     order, quotients through the diagonals' reciprocals:
+ *                     stored coefficients, and constant ones.
+ *   k_level_cluster, k_level_cluster_x
+ *                     all the sweeps of a level of 64^2 to 256^2 (FP32) or
+ *                     64^2 and 128^2 (FP64) in one thread-block cluster, a
+ *                     strip of the level in each CTA's shared memory.
  *   k_bottom          the coarse end of the cycle in one single-CTA launch:
  *                     restriction of res down to minlevel, the coarsest zero,
  *                     then for each level up to a small one the bilinear
@@ -203,23 +210,12 @@ __device__ __forceinline__ void put_quad (T * a0, T * a1, int off, const Quad<T>
   *(T2 *) (a1 + off) = o;
 }
 
-/* The bilinear prolongation (multigrid-common.h:124-140) of fine cell
-   (i, j) from the coarse level c (geometry gc, ghosts filled), with
-   k_prolong2d_blk's expression and order, so that a tile launch that
-   stages it instead of the iterate gives the values the prolongation
-   launch would have written (bit-identical in FP64). */
-template <typename T>
-__device__ __forceinline__ T prolong_cell (const T * __restrict__ c, const bmg_geom & gc, int i, int j)
-{
-  const int ci = i >> 1, cj = j >> 1, cx = (i & 1) ? 1 : -1, cy = (j & 1) ? 1 : -1;
-  const T m = c[cidx<2> (gc, ci, cj, 0)], mx = c[cidx<2> (gc, ci + cx, cj, 0)];
-  const T my = c[cidx<2> (gc, ci, cj + cy, 0)], mxy = c[cidx<2> (gc, ci + cx, cj + cy, 0)];
-  return (T(9)*m + T(3)*(mx + my) + mxy)/T(16);
-}
-
-/* the same for the K fine cells (i, j0) .. (i, j0 + K - 1) of one row, j0
-   even: the K/2 + 2 coarse values of the two coarse rows involved read
-   once */
+/* The bilinear prolongation (multigrid-common.h:124-140) of the K fine cells
+   (i, j0) .. (i, j0 + K - 1) of one row, j0 even, from the coarse level c
+   (geometry gc, ghosts filled): the K/2 + 2 coarse values of the two coarse
+   rows involved read once.  k_prolong2d_blk's expression and order, so that a
+   tile launch that stages it instead of the iterate gives the values the
+   prolongation launch would have written (bit-identical in FP64). */
 template <typename T, int K>
 __device__ __forceinline__ void prolong_row (const T * __restrict__ c, const bmg_geom & gc, int i, int j0,
                                              T * v)
@@ -601,11 +597,6 @@ __device__ __forceinline__ void sts_f4 (unsigned a, float4 v)
 {
   asm volatile ("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
                 :: "r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-
-__device__ __forceinline__ void sts_f1 (unsigned a, float v)
-{
-  asm volatile ("st.shared.f32 [%0], %1;" :: "r"(a), "f"(v) : "memory");
 }
 
 template <int TS, bool LAM, bool BOX>
@@ -1158,11 +1149,6 @@ __device__ __forceinline__ double lds_d1 (unsigned a)
 __device__ __forceinline__ void sts_d2 (unsigned a, double2 v)
 {
   asm volatile ("st.shared.v2.f64 [%0], {%1, %2};" :: "r"(a), "d"(v.x), "d"(v.y) : "memory");
-}
-
-__device__ __forceinline__ void sts_d1 (unsigned a, double v)
-{
-  asm volatile ("st.shared.f64 [%0], %1;" :: "r"(a), "d"(v) : "memory");
 }
 
 /* The plain FP64 form of k_relax_tile2d_w on large levels: the same
@@ -2164,24 +2150,6 @@ __device__ __forceinline__ void bot_pass2d (const bmg_geom & g, T * a, const T *
   }
 }
 
-template <typename T>
-__device__ __forceinline__ void bot_pass2d_any (const bmg_geom & g, void * dav, const void * resv,
-                                const void * const * al, const BotLevel & L, const void * lamp,
-                                const BCH & bc, int color, int nt)
-{
-  T * a = (T *) dav;
-  const T * b = (const T *) resv;
-  const T * ax = (const T *) al[0], * ay = (const T *) al[1], * lam = (const T *) lamp;
-  const T axc = (T) L.alpha[0].c, ayc = (T) L.alpha[1].c, lamc = (T) L.lambda.c;
-  const T D2 = (T) L.Delta*(T) L.Delta;
-  if ((ax == NULL) != (ay == NULL))   /* one component stored, one constant */
-    bot_pass<2, T> (g, dav, resv, al, L, lamp, bc, color, 0, nt);
-  else if (ax && lam) bot_pass2d<T, true, true, 1> (g, a, b, ax, ay, axc, ayc, lam, lamc, D2, bc, color, nt);
-  else if (ax) bot_pass2d<T, true, false, 1> (g, a, b, ax, ay, axc, ayc, lam, lamc, D2, bc, color, nt);
-  else if (lam) bot_pass2d<T, false, true, 1> (g, a, b, ax, ay, axc, ayc, lam, lamc, D2, bc, color, nt);
-  else bot_pass2d<T, false, false, 1> (g, a, b, ax, ay, axc, ayc, lam, lamc, D2, bc, color, nt);
-}
-
 /* all nrelax sweeps of one 2D level, every parameter in registers (the
    per-level parameters live in the kernel's parameter space, and reading
    them inside the sweep loop costs a constant-cache miss per pass) */
@@ -2318,8 +2286,7 @@ template <typename T, int K>
 __device__ __forceinline__ void bot_sweeps2d_reg (const bmg_geom g, T * a, const T * b,
                                                   const T * ax, const T * ay, T axc,
                                                   T ayc, const T * lam, T lamc,
-                                                  T D2, const BCH bc, int nrelax, int nt,
-                                                  bool small)
+                                                  T D2, const BCH bc, int nrelax, int nt)
 {
   const int n = g.n, P = g.P, nh = n >> 1, total = n*nh;
   const int lh = 30 - __clz (n);              /* log2 (n) - 1 */
@@ -2387,8 +2354,7 @@ __device__ __forceinline__ void bot_sweeps2d_reg (const bmg_geom g, T * a, const
             if ((w & 3) == 3) a[e[k] + ro + co] = (w & 4) ? -vi : vi;
           }
         }
-      if (small) __syncwarp ();
-      else __syncthreads ();
+      __syncthreads ();
     }
 }
 
@@ -2403,13 +2369,13 @@ __device__ __forceinline__ void bot_level2d (const bmg_geom g, void * dav, const
   const T * b = (const T *) resv, * ax = (const T *) axv, * ay = (const T *) ayv,
     * lam = (const T *) lamv;
   const T D2 = (T) Delta*(T) Delta;
-  /* up to four cells per colour per thread in FP32, two in FP64
-     (registers) */
-  constexpr int K = sizeof (T) == 4 ? 4 : 2;
-  if (fast && g.n >= 2 && g.n*(g.n >> 1) <= K*nt) {
-    bot_sweeps2d_reg<T, K> (g, a, b, ax, ay, (T) axc, (T) ayc, lam, (T) lamc, D2, bc, nrelax, nt, small);
-    return;
-  }
+  /* four cells per colour and thread: an FP32 level of 64^2 (in FP64 two
+     would hold no level that bot_sweeps_own does not) */
+  if constexpr (sizeof (T) == 4)
+    if (fast && g.n >= 2 && g.n*(g.n >> 1) <= 4*nt) {
+      bot_sweeps2d_reg<T, 4> (g, a, b, ax, ay, (T) axc, (T) ayc, lam, (T) lamc, D2, bc, nrelax, nt);
+      return;
+    }
   if (ax && lam)
     bot_sweeps2d<T, true, true> (g, a, b, ax, ay, (T) axc, (T) ayc, lam, (T) lamc, D2, bc, nrelax, nt, small);
   else if (ax)
@@ -2527,8 +2493,9 @@ __global__ void __launch_bounds__ (BOT_THREADS, 1) k_bottom (const __grid_consta
       bot_prolong_st<DIM> (P.lv[m - 1].st, P.sm[m - 1].gs, sm_at (bsm, P.sm[m - 1].off_da),
                            L.st, S.gs, da, P.bc, 0);
     __syncthreads ();
-    /* levels of at most BOT_WARP_CELLS cells are relaxed by warp 0 alone,
-       with warp barriers; the other warps wait at the level's end */
+    /* levels of at most BOT_WARP_CELLS cells (in one dimension; in two and
+       three the single cell, which bot_own_level leaves) are relaxed by warp
+       0 alone, with warp barriers; the other warps wait at the level's end */
     const bool small = gs.size <= BOT_WARP_CELLS;
     const int nt = small ? 32 : blockDim.x, nrelax = P.nrelax, st = L.st;
     if (DIM == 2 && (al[0] == NULL) == (al[1] == NULL)) {
