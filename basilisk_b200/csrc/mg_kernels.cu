@@ -121,8 +121,10 @@ __global__ void k_relax3_pair (bmg_geom g, T * out, const T * in, const T * __re
   }
   const T v = nn/d;
   out[id] = v;
-  /* the shorter code where FP64 levels are bound by HBM (256^3: 33.7 -> 32.1
-     us per pass) */
+  /* the shorter code in FP64, for the level that HBM bounds.  us per sweep
+     with ghosts_homog_any / ghosts_homog: 16^3 8.2 / 7.7, 32^3 8.2 / 7.7,
+     64^3 11.3 / 10.4, 128^3 50.4 / 48.2, 256^3 356 / 367, where a solve
+     spends its time */
   if (sizeof (T) == 8) ghosts_homog_any<3, T> (out, g, i, j, 2*q + o, v, bc);
   else ghosts_homog<3, T> (out, g, i, j, 2*q + o, v, bc);
   if (COR) {

@@ -31,14 +31,17 @@
  * a single block.
  *
  * The solve is the reference's mg_solve / mg_cycle (poisson.h:32-90,
- * 139-235) with one relaxation pass per launch (the coarse levels in one
- * launch of one CTA) and the boundary with each pass, exactly where the
- * single-grid solve has one: the
- * zero or prolonged correction of a level, each colour pass of a red-black
- * sweep (red, boundary, black, boundary) or each Jacobi sweep, and a after
- * the correction a += da.  Every value is computed by the kernels the
- * single-grid solve uses, in the same order, so a decomposed solve gives
- * the single grid's solution bit for bit (FP64) when the single grid's
+ * 139-235).  On one device the coarse levels of a red-black cycle are one
+ * launch of one CTA; in two dimensions the middle levels take several sweeps
+ * per launch, on tiles whose windows reach into the neighbouring blocks; the
+ * others, Jacobi sweeps and the other dimensions take a pass per launch.  A
+ * boundary stands where the single-grid solve has one: with the zero or
+ * prolonged correction of a level, each colour pass (red, boundary, black,
+ * boundary) or Jacobi sweep -- inside a tile or CTA as the neighbours' cells
+ * themselves, written as images by the launch's end -- and with a after the
+ * correction a += da.  mg_blocks.cu's kernels compute every value in the
+ * expressions and order of the single-grid kernels, so a decomposed solve
+ * gives the single grid's solution bit for bit (FP64) when the single grid's
  * minlevel is the blocks' minlevel plus log2 (dims[0]); mgstats.sum is the
  * sum of the blocks' sums, a reduction in another order.
  */

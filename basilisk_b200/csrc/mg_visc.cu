@@ -308,7 +308,8 @@ struct VBotParams {
    the coefficients of a thread's cells (one of each colour) in registers.
    As one launch per pass these levels cost six to eight launches of 3 to
    5 us per sweep and level for a few hundred cells.  Bound: the latency of
-   one update (two divisions, two barriers) per pass. */
+   one update (its sum, a quotient through the reciprocal of the denominator,
+   two barriers) per pass. */
 template <int DIM>
 __global__ void __launch_bounds__ (VB_THREADS, 1) k_visc_bottom (const __grid_constant__ VBotParams P)
 {
