@@ -90,7 +90,7 @@ struct bmg_tree {
   span_t sched[2][TMAX + 1];
   bmg_tree_rule * dsrules;
   /* the correction's boundary of each level by dependence: spans of deps,
-     whose cells and rules live in ddlist and ddrules */
+     whose cells and rules live in ddlist and ddrules (one allocation) */
   tdep * deps;
   span_t dep[TMAX + 1];
   uint32_t * ddlist;
@@ -98,7 +98,7 @@ struct bmg_tree {
   /* the cycle in distributed shared memory (mg_tree_cycle.cu); tc.slots = 0:
      none for this tree */
   bmg_tc tc;
-  void * dtc[4];                      /* its device arrays: levels, own, id, src */
+  void * dtc;                         /* its device arrays: levels, src, own, id */
   bmg_tree_levels T;
   double * dpart;
   int npart;
@@ -146,8 +146,7 @@ static void tree_release (struct bmg_tree * t)
   for (int i = 0; i < NTGRAPH; i++) graph_drop (&t->graphs[i]);
   for (int l = 0; l <= TMAX; l++) { free (t->fl[l]); free (t->nb[l]); }
   cudaFree (t->dflags); cudaFree (t->dlist); cudaFree (t->drules); cudaFree (t->dpart);
-  cudaFree (t->dsrules); cudaFree (t->ws32); cudaFree (t->ddlist); cudaFree (t->ddrules);
-  for (int k = 0; k < 4; k++) cudaFree (t->dtc[k]);
+  cudaFree (t->dsrules); cudaFree (t->ws32); cudaFree (t->ddrules); cudaFree (t->dtc);
   free (t->stages); free (t->deps);
   free (t);
 }
@@ -438,6 +437,14 @@ static int dep_visit (depset * s, int m, int i, int j)
   return dep_mark (s, mk, m, i, j, d + 1);
 }
 
+/* whether the tree's cells may fit some form's slots */
+static int cycle_wanted (const struct bmg_tree * t)
+{
+  long active = 0;
+  for (int l = 0; l <= t->depth; l++) active += t->act[l].n;
+  return t->interp && !t->no_cycle && active <= (long) BMG_TC_RANKS*BMG_TC_SLOTS;
+}
+
 /* The records of the cycle in distributed shared memory: a slot of one of
    the ranks for every cell of the correction, dealt out evenly and in order
    by level, colour and kind (so that every level's relaxation set, its own
@@ -451,25 +458,28 @@ static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h
 {
   const int D = t->depth, NR = BMG_TC_RANKS;
   memset (&t->tc, 0, sizeof t->tc);
-  for (int k = 0; k < 4; k++) { cudaFree (t->dtc[k]); t->dtc[k] = NULL; }
-  long total = 0, active = 0;
+  cudaFree (t->dtc); t->dtc = NULL;
+  long total = 0;
   for (int l = 0; l <= D; l++) {
     if (t->dep[l].n > BMG_TC_STAGES) return;
     total += t->act[l].n + t->rl[l].n;
-    active += t->act[l].n;
     for (long k = 0; k < t->dep[l].n; k++) {
       const tdep * d = &t->deps[t->dep[l].off + k];
       total += d->nrest + d->nhalo + d->rules.n;
     }
   }
-  if (!t->interp || t->no_cycle || active > (long) NR*BMG_TC_SLOTS) return;
+  if (!cycle_wanted (t)) return;
   int err = 0;
   uint32_t * slot[TMAX + 1], next[BMG_TC_RANKS];
   memset (slot, 0, sizeof slot);
-  bmg_tc_level * lv = calloc (D + 1, sizeof *lv);
-  uint32_t * own = malloc ((total + 1)*sizeof (uint32_t)), * id = calloc (total + 1, sizeof (uint32_t));
-  uint32_t * src = malloc ((total + 1)*4*sizeof (uint32_t));
-  if (!lv || !own || !id || !src) err = 1;
+  const size_t osrc = ((D + 1)*sizeof (bmg_tc_level) + 15)/16*16, oown = osrc + total*4*sizeof (uint32_t);
+  const size_t oid = oown + total*sizeof (uint32_t), bytes = oid + total*sizeof (uint32_t);
+  char * rec = malloc (bytes);
+  if (!rec) return;
+  memset (rec, 0, osrc);
+  memset (rec + oid, 0, bytes - oid);
+  bmg_tc_level * lv = (bmg_tc_level *) rec;
+  uint32_t * src = (uint32_t *) (rec + osrc), * own = (uint32_t *) (rec + oown), * id = (uint32_t *) (rec + oid);
   for (int l = 0; l <= D && !err; l++)
     if (!(slot[l] = calloc ((size_t) ((1 << l) + 2)*((1 << l) + 2), sizeof (uint32_t)))) err = 1;
   for (int r = 0; r < NR; r++) next[r] = 1;             /* offset 0: a zero */
@@ -477,25 +487,27 @@ static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h
 #define CI(e) ((int) (((e) >> 14) & 0x3FFF) - 1)
 #define CJ(e) ((int) ((e) & 0x3FFF) - 1)
 #define SLOT(e) slot[LVL (e)][HX (LVL (e), CI (e), CJ (e))]
-  /* active cells: red leaves, black leaves, red refined, black refined */
-  for (int l = 0; l <= D && !err; l++)
-    for (int kind = 0; kind < 4; kind++) {
-      long n = 0, k;
-      for (int pass = 0; pass < 2; pass++) {
-        k = 0;
-        for (long q = 0; q < t->act[l].n; q++) {
-          const uint32_t e = h[t->act[l].off + q];
-          const int leaf = (t->fl[l][HX (l, CI (e), CJ (e))] & BMG_T_LEAF) != 0;
-          if (((CI (e) + CJ (e)) & 1) != (kind & 1) || leaf != !(kind & 2)) continue;
-          if (pass == 1) {
-            const uint32_t r = (uint32_t) (k*NR/n);
-            SLOT (e) = r << 16 | (next[r]++ & 0xffff);
-          }
-          k++;
-        }
-        n = k;
+  /* active cells: red leaves, black leaves, red refined, black refined, each
+     kind's k-th of n cells on rank k NR/n */
+  for (int l = 0; l <= D && !err; l++) {
+    const uint32_t * cells = h + t->act[l].off;
+#define KIND(e) (((CI (e) + CJ (e)) & 1) | (t->fl[l][HX (l, CI (e), CJ (e))] & BMG_T_LEAF ? 0 : 2))
+    long n[4] = {0, 0, 0, 0}, k[4] = {0, 0, 0, 0};
+    uint32_t at[4][BMG_TC_RANKS];
+    for (long q = 0; q < t->act[l].n; q++) n[KIND (cells[q])]++;
+    for (int kind = 0; kind < 4; kind++)
+      for (long r = 0; r < NR; r++) {
+        at[kind][r] = next[r];
+        next[r] += (uint32_t) (((r + 1)*n[kind] + NR - 1)/NR - (r*n[kind] + NR - 1)/NR);
       }
+    for (long q = 0; q < t->act[l].n; q++) {
+      const uint32_t e = cells[q];
+      const int kind = KIND (e);
+      const uint32_t r = (uint32_t) (k[kind]++*NR/n[kind]);
+      SLOT (e) = r << 16 | (at[kind][r]++ & 0xffff);
     }
+#undef KIND
+  }
   /* the other cells of the stages, from the finest level's down */
   for (int l = D; l >= 0 && !err; l--)
     for (long d = 0; d < t->dep[l].n; d++) {
@@ -587,19 +599,20 @@ static void cycle_records (bmg_grid * g, struct bmg_tree * t, const uint32_t * h
 #undef LVL
 #undef CI
 #undef CJ
-  const size_t sz[4] = {(D + 1)*sizeof *lv, total*sizeof (uint32_t), total*sizeof (uint32_t), total*4*sizeof (uint32_t)};
-  const void * hp[4] = {lv, own, id, src};
-  for (int k = 0; k < 4 && !err; k++)
-    if (cudaMalloc (&t->dtc[k], sz[k] + 16) != cudaSuccess ||
-        cudaMemcpy (t->dtc[k], hp[k], sz[k], cudaMemcpyHostToDevice) != cudaSuccess) err = 1;
-  t->tc.lv = t->dtc[0]; t->tc.own = t->dtc[1]; t->tc.id = t->dtc[2]; t->tc.src = t->dtc[3];
+  if (!err && (cudaMalloc (&t->dtc, bytes) != cudaSuccess ||
+               cudaMemcpy (t->dtc, rec, bytes, cudaMemcpyHostToDevice) != cudaSuccess)) err = 1;
   if (err) {
     cudaGetLastError ();
-    for (int k = 0; k < 4; k++) { cudaFree (t->dtc[k]); t->dtc[k] = NULL; }
+    cudaFree (t->dtc); t->dtc = NULL;
     memset (&t->tc, 0, sizeof t->tc);
   }
+  else {
+    const char * d = t->dtc;
+    t->tc.lv = (const bmg_tc_level *) d; t->tc.src = (const uint32_t *) (d + osrc);
+    t->tc.own = (const uint32_t *) (d + oown); t->tc.id = (const uint32_t *) (d + oid);
+  }
   for (int l = 0; l <= D; l++) free (slot[l]);
-  free (lv); free (own); free (id); free (src);
+  free (rec);
 }
 
 /* a cell that a pass reads (most are in the set) */
@@ -618,6 +631,14 @@ static int depend (bmg_grid * g, struct bmg_tree * t, const uint32_t * h)
   bmg_tree_rule * rules = NULL;
   long nlist = 0, nrules = 0, caplist = 0, caprules = 0, ndeps = 0, capdeps = 0;
   free (t->deps); t->deps = NULL;
+  cudaFree (t->ddrules);
+  t->ddlist = NULL; t->ddrules = NULL;
+  /* (a full tree's boundary is its box ghosts, interpreted as such) */
+  if (t->full && !cycle_wanted (t)) {
+    for (int l = 0; l <= t->depth; l++) t->dep[l].off = t->dep[l].n = 0;
+    cycle_records (g, t, h, NULL, NULL);
+    return BMG_OK;
+  }
   for (int l = 0; l <= t->depth && !s.err; l++) {
     const size_t m = (size_t) ((1 << l) + 2)*((1 << l) + 2);
     if (!(s.mark[l] = calloc (m, 1))) s.err = 1;
@@ -688,15 +709,18 @@ static int depend (bmg_grid * g, struct bmg_tree * t, const uint32_t * h)
   }
   for (int l = 0; l <= t->depth; l++) free (s.mark[l]);
   free (s.cell);
-  cudaFree (t->ddlist); cudaFree (t->ddrules);
-  t->ddlist = NULL; t->ddrules = NULL;
-  if (!s.err &&
-      (cudaMalloc ((void **) &t->ddlist, (nlist + 1)*sizeof (uint32_t)) != cudaSuccess ||
-       cudaMalloc ((void **) &t->ddrules, (nrules + 1)*sizeof (bmg_tree_rule)) != cudaSuccess ||
-       (nlist && cudaMemcpy (t->ddlist, list, nlist*sizeof (uint32_t), cudaMemcpyHostToDevice) != cudaSuccess) ||
-       (nrules && cudaMemcpy (t->ddrules, rules, nrules*sizeof (bmg_tree_rule), cudaMemcpyHostToDevice)
-        != cudaSuccess)))
+  const size_t rb = nrules*sizeof (bmg_tree_rule), lb = nlist*sizeof (uint32_t);
+  char * both = s.err || t->full ? NULL : malloc (rb + lb + 1);
+  if (both) {
+    if (rb) memcpy (both, rules, rb);
+    if (lb) memcpy (both + rb, list, lb);
+  }
+  if (!s.err && !t->full &&
+      (!both || cudaMalloc ((void **) &t->ddrules, rb + lb + 1) != cudaSuccess ||
+       (rb + lb && cudaMemcpy (t->ddrules, both, rb + lb, cudaMemcpyHostToDevice) != cudaSuccess)))
     s.err = 1;
+  if (t->ddrules) t->ddlist = (uint32_t *) ((char *) t->ddrules + rb);
+  free (both);
   if (!s.err) cycle_records (g, t, h, list, rules);
   free (list); free (rules);
   return s.err ? BMG_ENOMEM : BMG_OK;
@@ -1118,6 +1142,7 @@ static void r_boundary (struct bmg_tree * t, opvec * o, int field, int l, int ho
 /* the boundary of da that a pass on level l reads, by dependence */
 static void r_depend (struct bmg_tree * t, opvec * o, int l)
 {
+  if (t->full) { r_boundary (t, o, F_DA, l, 1, SCHED_PRUNED); return; }
   for (long k = 0; k < t->dep[l].n; k++) {
     const tdep * d = &t->deps[t->dep[l].off + k];
     if (d->nrest + d->nhalo + d->rules.n > 0)
@@ -1183,9 +1208,12 @@ static int read_max (bmg_grid * g, double * m)
 /* whether the cycle runs in distributed shared memory: red-black, to the
    tree's depth, and the correction's cells fit.  The depth-10 band tree
    takes 140 ms per solve this way and 284 ms as interpreted
-   operations. */
+   operations.  A full tree's few passes are not worth the two more launches
+   (nrelax 1, depth 2: 206 us interpreted, 218 in three launches; 16 passes
+   and more: as fast at depth 2, 1.1 times at depth 7). */
 static int cycle_fits (const bmg_grid * g, const struct bmg_tree * t, const tkey * key)
 {
+  if (t->full && 2*key->nrelax*(key->maxlevel - key->minlevel + 1) < 16) return 0;
   return g->relax == BMG_RELAX_RBGS && t->tc.slots > 0 && key->nrelax > 0 &&
     key->minlevel <= key->maxlevel && key->maxlevel == t->depth && bmg_tree_cycle_fits (&t->tc, key->mixed);
 }

@@ -76,6 +76,12 @@ def same(one, other):
         np.testing.assert_array_equal(u, v)
 
 
+def few_passes(depth, shape):
+    """Full trees of one or two levels at nrelax 4 and below are interpreted
+    (depth 1 from minlevel 1)."""
+    return shape == "uniform" and depth < 2
+
+
 TREES = [(0, "uniform", 0, 0), (1, "uniform", 0, 0), (5, "uniform", 0, 0), (4, "corner", 0, 1),
          (8, "corner", 3, 0), (6, "band", 0, 0), (9, "band", 0, 0), (9, "band", 6, 2),
          (5, "random", 0, 0), (7, "random", 0, 0), (9, "random", 2, 3)]
@@ -87,7 +93,7 @@ def test_cycle_bit_identical_to_launches(depth, shape, minlevel, nrelax):
     interpreted = solve(depth, shape, minlevel, nrelax, "BMG_NO_TREE_CYCLE")
     same(fast, interpreted)
     same(fast, solve(depth, shape, minlevel, nrelax, "BMG_NO_TREE_INTERP"))
-    fits = shape != "half"
+    fits = shape != "half" and not few_passes(depth, shape)
     assert fast[0]["launches"] - interpreted[0]["launches"] == (2 * fast[0]["i"] if fits else 0)
 
 
@@ -96,4 +102,5 @@ def test_mixed_cycle_bit_identical_to_the_interpreter(depth, shape, minlevel, nr
     fast = solve(depth, shape, minlevel, nrelax, precision="mixed")
     interpreted = solve(depth, shape, minlevel, nrelax, "BMG_NO_TREE_CYCLE", precision="mixed")
     same(fast, interpreted)
-    assert fast[0]["launches"] - interpreted[0]["launches"] == 2 * fast[0]["i"] > 0
+    fits = not few_passes(depth, shape)
+    assert fast[0]["launches"] - interpreted[0]["launches"] == (2 * fast[0]["i"] if fits else 0)

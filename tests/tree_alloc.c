@@ -48,17 +48,14 @@ int main (void)
   g.off64[g.depth + 1] = off;
   int depth = 5;
   if (bmg_tree_refine (&g, corner, &depth) <= 0 || g.tree->tc.slots <= 0) return 2;
-  int first = 0;
-  for (int k = 1; k <= count; k++) if (given[k] == g.tree->dtc[0]) first = k;
+  int records = 0;
+  for (int k = 1; k <= count; k++) if (given[k] == g.tree->dtc) records = k;
   bmg_tree_free (&g);
-  for (int k = first; k < first + 4; k++) {
-    count = 0;
-    fail_at = k;
-    const int cells = bmg_tree_refine (&g, corner, &depth);
-    if (cells <= 0 || !g.tree) { printf ("refining without memory for the records: %d\n", cells); return 4; }
-    if (g.tree->tc.slots || g.tree->dtc[0]) return 5;
-    if (k < first + 3) bmg_tree_free (&g);
-  }
+  count = 0;
+  fail_at = records;
+  const int cells = bmg_tree_refine (&g, corner, &depth);
+  if (cells <= 0 || !g.tree) { printf ("refining without memory for the records: %d\n", cells); return 4; }
+  if (g.tree->tc.slots || g.tree->dtc) return 5;
   fail_at = 0;
   depth = 6;
   if (bmg_tree_refine (&g, corner, &depth) <= 0 || g.tree->tc.slots <= 0) return 6;
