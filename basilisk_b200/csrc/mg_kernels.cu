@@ -625,13 +625,21 @@ struct Row {
   }
 };
 
-/* extents of the compact array as rows: nr rows of nk */
+/* extents of the compact array as rows: nr rows of nk.  In 3D, whose levels
+   have rows enough, a row takes as few threads as reach its end with ROWU
+   elements each, so that a thread has several loads in flight (us per set of
+   the faces / get of the cells, 128 threads per row -> so: 128^3 120 / 36 ->
+   104 / 28, 256^3 264 / 82 -> 218 / 67; one thread per element: 112 / 34 and
+   275 / 90); in 2D that leaves too few blocks on small levels (256^2 with
+   ghosts 33 -> 36 us) and changes nothing on large ones */
 template <int DIM>
 void row_launch (int ni, int nj, int nk, int & len, dim3 & grid, dim3 & block)
 {
   len = DIM == 1 ? ni : DIM == 2 ? nj : nk;
   const long long rows = DIM == 1 ? 1 : DIM == 2 ? ni : (long long) ni*nj;
-  const int bx = len >= 128 ? 128 : len >= 64 ? 64 : 32, by = 256/bx;
+  const int bx = DIM == 3 ? (len <= 32*ROWU ? 32 : len <= 64*ROWU ? 64 : 128)
+    : len >= 128 ? 128 : len >= 64 ? 64 : 32;
+  const int by = 256/bx;
   block = dim3 (bx, by, 1);
   grid = dim3 ((unsigned) ((rows + by - 1)/by), (len + bx*ROWU - 1)/(bx*ROWU), 1);
 }
