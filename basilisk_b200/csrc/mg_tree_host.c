@@ -733,26 +733,40 @@ static int derive (bmg_grid * g, struct bmg_tree * t)
   const int D = t->depth;
   long nact[TMAX + 1] = {0}, nref[TMAX + 1] = {0}, nprol[TMAX + 1] = {0}, nleaf[TMAX + 1] = {0};
   long long leaves = 0;
+  /* the active cells, level by level, in the one pass over the dense levels */
+  uint32_t * active = NULL;
+  long n = 0, room = 0;
   for (int l = 0; l <= t->hmax; l++) {
-    const size_t m = (size_t) ((1 << l) + 2)*((1 << l) + 2);
-    for (size_t k = 0; k < m; k++) t->fl[l][k] &= ~(BMG_T_HALO | BMG_T_PROL);
-  }
-  for (int l = 0; l <= D; l++) {
-    const int n = 1 << l;
-    for (int i = 0; i < n; i++)
-      for (int j = 0; j < n; j++) {
-        unsigned char * f = &t->fl[l][HX (l, i, j)];
-        if (!(*f & BMG_T_ACTIVE)) continue;
-        nact[l]++;
-        if (!(*f & BMG_T_LEAF)) { nref[l]++; continue; }
-        nleaf[l]++; leaves++;
-        if (t->nb[l][HX (l, i, j)] > 0) {
-          *f |= BMG_T_PROL;
-          nprol[l]++;
-          for (int c = 0; c < 4; c++)
-            t->fl[l + 1][HX (l + 1, 2*i + (c >> 1), 2*j + (c & 1))] |= BMG_T_HALO;
-        }
+    const int nl = 1 << l;
+    const long first = n;
+    for (int i = -1; i <= nl; i++) {
+      unsigned char * f = &t->fl[l][HX (l, i, 0)];
+      for (int j = -1; j <= nl; j++) f[j] &= ~(BMG_T_HALO | BMG_T_PROL);
+      if (i < 0 || i >= nl || l > D) continue;
+      if (n + nl > room) {
+        room = 2*room + nl;
+        uint32_t * q = realloc (active, room*sizeof (uint32_t));
+        if (!q) { free (active); return FAIL (BMG_ENOMEM); }
+        active = q;
       }
+      for (int j = 0; j < nl; j++)
+        if (f[j] & BMG_T_ACTIVE) active[n++] = pack (l, i, j);
+    }
+    if (l <= D) nact[l] = n - first;
+  }
+#define CI(e) ((int) (((e) >> 14) & 0x3FFF) - 1)
+#define CJ(e) ((int) ((e) & 0x3FFF) - 1)
+  for (long k = 0; k < n; k++) {
+    const int l = (int) (active[k] >> 28), i = CI (active[k]), j = CJ (active[k]);
+    unsigned char * f = &t->fl[l][HX (l, i, j)];
+    if (!(*f & BMG_T_LEAF)) { nref[l]++; continue; }
+    nleaf[l]++; leaves++;
+    if (t->nb[l][HX (l, i, j)] > 0) {
+      *f |= BMG_T_PROL;
+      nprol[l]++;
+      for (int c = 0; c < 4; c++)
+        t->fl[l + 1][HX (l + 1, 2*i + (c >> 1), 2*j + (c & 1))] |= BMG_T_HALO;
+    }
   }
   t->nleaves = leaves;
   t->full = leaves == (1LL << (2*D));
@@ -771,39 +785,35 @@ static int derive (bmg_grid * g, struct bmg_tree * t)
     below += nleaf[l];
   }
   uint32_t * h = malloc ((total + 1)*sizeof (uint32_t));
-  if (!h) return FAIL (BMG_ENOMEM);
+  if (!h) { free (active); return FAIL (BMG_ENOMEM); }
   long pa[TMAX + 1], pr[TMAX + 1], pp[TMAX + 1], pl = t->leaves.off;
   for (int l = 0; l <= D; l++) { pa[l] = t->act[l].off; pr[l] = t->ref[l].off; pp[l] = t->prol[l].off; }
-  for (int l = 0; l <= D; l++) {
-    const int n = 1 << l;
-    for (int i = 0; i < n; i++)
-      for (int j = 0; j < n; j++) {
-        const unsigned char f = t->fl[l][HX (l, i, j)];
-        if (!(f & BMG_T_ACTIVE)) continue;
-        const uint32_t e = pack (l, i, j);
-        h[pa[l]++] = e;
-        if (!(f & BMG_T_LEAF)) h[pr[l]++] = e;
-        else {
-          h[pl++] = e;
-          if (f & BMG_T_PROL) h[pp[l]++] = e;
-        }
-      }
+  for (long k = 0; k < n; k++) {
+    const uint32_t e = active[k];
+    const int l = (int) (e >> 28);
+    const unsigned char f = t->fl[l][HX (l, CI (e), CJ (e))];
+    h[pa[l]++] = e;
+    if (!(f & BMG_T_LEAF)) h[pr[l]++] = e;
+    else {
+      h[pl++] = e;
+      if (f & BMG_T_PROL) h[pp[l]++] = e;
+    }
   }
+  free (active);
+#undef CI
+#undef CJ
   /* relax set of level l (foreach_level_or_leaf): its active cells and the
      leaves below, red first */
   for (int l = 0; l <= D; l++) {
     long w = t->rl[l].off;
     for (int c = 0; c < 2; c++) {
       if (c == 1) t->rl1[l] = w - t->rl[l].off;
-      for (int m = l; m >= 0; m--) {
-        const int n = 1 << m;
-        for (int i = 0; i < n; i++)
-          for (int j = 0; j < n; j++) {
-            const unsigned char f = t->fl[m][HX (m, i, j)];
-            if (!(f & BMG_T_ACTIVE) || (m < l && !(f & BMG_T_LEAF)) || ((i + j) & 1) != c) continue;
-            h[w++] = pack (m, i, j);
-          }
-      }
+      for (int m = l; m >= 0; m--)
+        for (long k = t->act[m].off; k < t->act[m].off + t->act[m].n; k++) {
+          const uint32_t e = h[k];
+          const int i = (int) ((e >> 14) & 0x3FFF) - 1, j = (int) (e & 0x3FFF) - 1;
+          if (((i + j) & 1) == c && (m == l || (t->fl[m][HX (m, i, j)] & BMG_T_LEAF))) h[w++] = e;
+        }
     }
   }
   /* ghost rules */
@@ -830,8 +840,7 @@ static int derive (bmg_grid * g, struct bmg_tree * t)
     const int n = 1 << l;
     const bmg_geom * gg = &g->g64[l];
     for (int i = -1; i <= n; i++)
-      for (int j = -1; j <= n; j++)
-        hf[g->off64[l] + (size_t) (i + 1)*gg->P + gg->xo + j] = t->fl[l][HX (l, i, j)];
+      memcpy (hf + g->off64[l] + (size_t) (i + 1)*gg->P + gg->xo - 1, &t->fl[l][HX (l, i, -1)], n + 2);
   }
   cudaFree (t->dflags); cudaFree (t->dlist); cudaFree (t->drules);
   t->dflags = NULL; t->dlist = NULL; t->drules = NULL;
